@@ -46,7 +46,8 @@ sys.path.insert(0, os.path.join(ROOT, "sparse-blas_b200"))
 import numpy as np  # noqa: E402
 
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0}
-KERNEL_TAGS = {1: "vector_kernel", 2: "merge_kernel", 3: "tiled_kernel", 5: "rows_kernel"}
+KERNEL_TAGS = {1: "vector_kernel", 2: "merge_kernel", 3: "tiled_kernel", 5: "rows_kernel",
+               6: "sliced_kernel"}
 
 
 def algo_bytes(m, n, nnz):

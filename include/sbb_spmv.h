@@ -93,6 +93,11 @@ enum {
                               batch classes' configurations on the GPU; the
                               parameters (21.6 KB) are copied to a device
                               the first time it is used and kept until exit */
+    SBB_KERNEL_SLICED = 6, /* K5: slices of 32/W rows, W lanes a row, from a
+                              copy of the matrix in the order a warp reads it;
+                              for short, even rows (vector_width: W = 1, 2, 4,
+                              8 or 16, 0 = from mean row length).  No
+                              counterpart in the reference. */
     SBB_KERNEL_ROWS = 5    /* K4: blocks of <= 32 rows and <= 384 nnz (rows
                               longer than 384 nnz split into pieces), staged
                               into shared memory by TMA straight from the

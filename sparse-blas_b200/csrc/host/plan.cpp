@@ -34,15 +34,29 @@ int plan_launches(const Plan *p)
         extern int rows_launches(const Plan *);
         return rows_launches(p);
     }
+    case SBB_KERNEL_SLICED: return 1;
     default: return 0;
     }
 }
 
 void launch_rowptr_check(const int *rp, int m, int nnz, unsigned *status, cudaStream_t s);
 
+// Lanes per row of the row slices: enough that a row takes about 8 to 32 steps
+// (us for 1, 2, 4, 8 lanes: rows of 6 11.8, 12.4, 15.7, -; of 24 15.5, 14.4,
+// 15.8, 19.0; of 50 -, 15.4, 15.0, 16.3; of 100 -, 27.1, 26.4, 26.6), and more
+// while the slices are fewer than an SM's warps times the SMs (3,000 rows of 24:
+// 5.3, 3.6, 2.8, 2.4).
+static int slice_width(int m, double mean)
+{
+    int w = mean <= 8 ? 1 : (mean <= 32 ? 2 : (mean <= 128 ? 4 : 8));
+    while (w < 8 && w < mean && (long long)m * w / 32 < 148 * 48) w <<= 1;
+    return w;
+}
+
 // Default (heuristic) kernel choice, the method without the learned selector:
-// vector CSR when rows are short and even, 32x4 tiles otherwise (the fastest
-// tile shape measured on the irregular benchmark matrices).
+// rows that are short and even for row slices or vector CSR, 32x4 tiles
+// otherwise (the fastest tile shape measured on the irregular benchmark
+// matrices).
 int default_kernel_choice(int m, int nnz, int max_row, int *vector_width, int *ipt, int *sigma)
 {
     double mean = m > 0 ? (double)nnz / m : 0.0;
@@ -114,6 +128,8 @@ static int dalloc(T **p, size_t count, cudaStream_t s, size_t *acc)
     return SBB_OK;
 }
 
+extern void sliced_free_async(Plan *, cudaStream_t);
+
 void plan_free_async(Plan *p, cudaStream_t s)
 {
     void *ptrs[] = {p->tile_row, p->tile_nnz, p->carry_val, p->queue, p->status};
@@ -124,6 +140,7 @@ void plan_free_async(Plan *p, cudaStream_t s)
     tiled_free_async(p, s);
     extern void rows_free_async(Plan *, cudaStream_t);
     rows_free_async(p, s);
+    sliced_free_async(p, s);
     p->tile_row = p->tile_nnz = nullptr;
     p->carry_val = nullptr;
     p->queue = p->status = nullptr;
@@ -139,6 +156,8 @@ void plan_free(Plan *p)
     tiled_free(p);
     extern void rows_free(Plan *);
     rows_free(p);
+    extern void sliced_free(Plan *);
+    sliced_free(p);
     p->tile_row = p->tile_nnz = nullptr;
     p->carry_val = nullptr;
     p->queue = p->status = nullptr;
@@ -147,9 +166,49 @@ void plan_free(Plan *p)
 extern int tiled_build(Plan *p, cudaStream_t s);
 extern int tiled_run(Plan *p, double alpha, const void *x, double beta, double *y,
                      cudaStream_t s);
+extern int sliced_build(Plan *p, cudaStream_t s);
+extern int sliced_run(Plan *p, double alpha, const void *x, double beta, double *y,
+                      cudaStream_t s);
 extern int rows_build(Plan *p, cudaStream_t s);
 extern int rows_run(Plan *p, double alpha, const void *x, double beta, double *y,
                     cudaStream_t s);
+
+// Rows that the slices suit: none longer than 4 times the power of two that the
+// mean row length rounds up to (the vector rule's bound, up to a mean of 128).
+static bool even_rows(int m, int nnz, int max_row)
+{
+    if (nnz <= 0 || m > kTiledMaxRows) return false;
+    long long v = 2;
+    while (v < 128 && v < (double)nnz / m) v <<= 1;
+    return max_row <= 4 * v;
+}
+
+// A validated plan of row slices, `width` lanes a row (0: by the mean row
+// length).  fall_back: 1 instead of an error when the copy does not fit or
+// finds a column out of range, for a caller whose other choice needs no copy
+// and reports such columns when it runs.
+static int build_sliced(Plan *p, int width, bool fall_back, cudaStream_t s)
+{
+    const int vw = p->vector_width;
+    const size_t bytes = p->scratch_bytes;
+    p->vector_width = width ? width : slice_width(p->m, p->m > 0 ? (double)p->nnz / p->m : 0.0);
+    int rc = sliced_build(p, s);
+    if (rc == SBB_OK) {
+        unsigned st = 0;
+        SBB_CUDA(cudaMemcpyAsync(&st, p->status, sizeof(st), cudaMemcpyDeviceToHost, s));
+        SBB_CUDA(cudaStreamSynchronize(s));
+        p->kernel = SBB_KERNEL_SLICED;
+        if (!(st & ST_BAD_COL)) return SBB_OK;
+        set_error("column index out of range [0, n)");
+        rc = SBB_ERR_INPUT;
+    }
+    if (!fall_back || rc == SBB_ERR_CUDA) return rc;
+    sliced_free_async(p, s);
+    p->vector_width = vw;
+    p->scratch_bytes = bytes;
+    SBB_CUDA(cudaMemsetAsync(p->status, 0, 4 * sizeof(unsigned), s));
+    return 1;
+}
 
 // Build scratch for the resolved kernel.  Validation (one sync) only when
 // `validate`; the drop-in validates while narrowing the row pointer instead.
@@ -204,6 +263,11 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
     int k = c.kernel;
     if (k == SBB_KERNEL_AUTO) {
         k = default_kernel_choice(p->m, p->nnz, want_stats ? p->max_row : INT_MAX, &vw, &ipt, &sigma);
+        if (want_stats && !p->lane32 && !c.vector_width && !c.tile_sigma &&
+            even_rows(p->m, p->nnz, p->max_row)) {
+            rc = build_sliced(p, 0, k == SBB_KERNEL_VECTOR, s);
+            if (rc <= 0) return rc;  // built, or an error that the choice below has too
+        }
         // FP32 storage: 32 x 8 tiles, which measured fastest for that form
         // (0.130 ms vs 0.166 ms for 32 x 4 on the 5.5M-row matrix)
         if (p->f32) sigma = 8;
@@ -271,6 +335,15 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
         }
         SBB_CUDA(cudaGetLastError());
         return SBB_OK;
+    }
+    if (k == SBB_KERNEL_SLICED) {
+        const int w = c.vector_width;
+        if (!validate || p->m > kTiledMaxRows || (w & (w - 1)) || w < 0 || w > 16) {
+            set_error("row slices need a validated plan of at most 2^31 - 1025 rows and "
+                      "vector_width 1, 2, 4, 8 or 16");
+            return SBB_ERR_ARG;
+        }
+        return build_sliced(p, w, false, s);
     }
     if (k == SBB_KERNEL_TILED) {
         rc = tiled_build(p, s);
@@ -359,6 +432,8 @@ int plan_run(Plan *p, double alpha, const void *x, double beta, double *y, cudaS
         return tiled_run(p, alpha, x, beta, y, s);
     case SBB_KERNEL_ROWS:
         return rows_run(p, alpha, x, beta, y, s);
+    case SBB_KERNEL_SLICED:
+        return sliced_run(p, alpha, x, beta, y, s);
     default:
         set_error("plan has no kernel");
         return SBB_ERR_ARG;

@@ -14,6 +14,34 @@ __device__ __forceinline__ double2 ld_stream(const double2 *p) { return __ldcs(p
 __device__ __forceinline__ float ld_stream(const float *p) { return __ldcs(p); }
 __device__ __forceinline__ float4 ld_stream(const float4 *p) { return __ldcs(p); }
 
+// The same loads, and the gather of x with an L2 policy, under a predicate and
+// without a branch: 0 where p is false (a branch per load would keep a lane's
+// loads from being in flight together).
+#define SBB_LOAD_IF(NAME, T, R, SZ, OP)                                                          \
+    __device__ __forceinline__ T NAME(const T *a, bool p)                                        \
+    {                                                                                            \
+        T v;                                                                                     \
+        asm("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n mov." SZ " %0, 0;\n @q " OP "." SZ         \
+            " %0, [%1];\n}" : "=" R(v) : "l"(a), "r"((int)p));                                   \
+        return v;                                                                                \
+    }
+#define SBB_KEEP_IF(T, R, SZ)                                                                    \
+    __device__ __forceinline__ T ld_keep_if(const T *a, bool p, uint64_t pol)                    \
+    {                                                                                            \
+        T v;                                                                                     \
+        asm("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n mov." SZ " %0, 0;\n"                     \
+            " @q ld.global.nc.L2::cache_hint." SZ " %0, [%1], %3;\n}"                             \
+            : "=" R(v) : "l"(a), "r"((int)p), "l"(pol));                                          \
+        return v;                                                                                \
+    }
+SBB_LOAD_IF(ld_stream_if, int, "r", "b32", "ld.global.cs")
+SBB_LOAD_IF(ld_stream_if, float, "f", "b32", "ld.global.cs")
+SBB_LOAD_IF(ld_stream_if, double, "d", "b64", "ld.global.cs")
+SBB_KEEP_IF(float, "f", "b32")
+SBB_KEEP_IF(double, "d", "b64")
+#undef SBB_LOAD_IF
+#undef SBB_KEEP_IF
+
 // x is gathered through the read-only path and kept in L2.
 template <typename T>
 __device__ __forceinline__ T ld_x(const T *p) { return __ldg(p); }
