@@ -32,26 +32,6 @@ struct Scratch {
     }
 };
 
-struct Acts {  // activations and error terms of N samples, carved from one block
-    float *xn, *h1, *h2, *y, *dy, *dz2, *dz1, *loss;
-    static size_t floats(int N)
-    {
-        return (size_t)N * (kMlpFeatures + 4 * kMlpHidden + 2 * kMlpClasses) + 32;
-    }
-    explicit Acts(float *base, int N)
-    {
-        float *p = base;
-        xn = p, p += (size_t)N * kMlpFeatures;
-        h1 = p, p += (size_t)N * kMlpHidden;
-        h2 = p, p += (size_t)N * kMlpHidden;
-        y = p, p += (size_t)N * kMlpClasses;
-        dy = p, p += (size_t)N * kMlpClasses;
-        dz2 = p, p += (size_t)N * kMlpHidden;
-        dz1 = p, p += (size_t)N * kMlpHidden;
-        loss = p;
-    }
-};
-
 // 1 / (classes * sum of sample weights), read back once (the weights are
 // fixed for a call).
 int inv_norm_of(const float *d_w, int N, cudaStream_t s, float *out)
@@ -105,8 +85,7 @@ int sbb_mlp_forward(const float *d_params, const float *d_x, int N, float *d_y, 
         set_error("bad sbb_mlp_forward arguments");
         return SBB_ERR_ARG;
     }
-    launch_mlp_forward(d_params, d_x, N, nullptr, nullptr, nullptr, d_y,
-                       static_cast<cudaStream_t>(stream));
+    launch_mlp_forward(d_params, d_x, N, d_y, static_cast<cudaStream_t>(stream));
     SBB_CUDA(cudaGetLastError());
     return SBB_OK;
 }
@@ -123,11 +102,8 @@ int sbb_mlp_grad(const float *d_params, const float *d_x, const float *d_t, cons
     int rc = inv_norm_of(d_w, N, s, &inv);
     if (rc != SBB_OK) return rc;
     Scratch mem(s);
-    if (!mem.get(sizeof(float) * Acts::floats(N))) return SBB_ERR_NOMEM;
-    Acts a(static_cast<float *>(mem.p), N);
-    launch_mlp_forward(d_params, d_x, N, a.xn, a.h1, a.h2, a.y, s);
-    launch_mlp_backward(d_params, N, a.xn, a.h1, a.h2, a.y, d_t, d_w, inv, a.dy, a.dz2, a.dz1,
-                        d_grad, d_loss, s);
+    if (!mem.get(sizeof(float) * mlp_parts_floats(N))) return SBB_ERR_NOMEM;
+    launch_mlp_grad(d_params, d_x, N, d_t, d_w, inv, static_cast<float *>(mem.p), d_grad, d_loss, s);
     SBB_CUDA(cudaGetLastError());
     return SBB_OK;
 }
@@ -144,17 +120,14 @@ int sbb_mlp_train(float *d_params, const float *d_x, const float *d_t, const flo
     int rc = inv_norm_of(d_w, N, s, &inv);
     if (rc != SBB_OK) return rc;
     Scratch mem(s);
-    if (!mem.get(sizeof(float) * (Acts::floats(N) + 3 * (size_t)kMlpParams))) return SBB_ERR_NOMEM;
-    Acts a(static_cast<float *>(mem.p), N);
-    float *g = static_cast<float *>(mem.p) + Acts::floats(N);
-    float *mo = g + kMlpParams, *vo = mo + kMlpParams;
+    if (!mem.get(sizeof(float) * (mlp_parts_floats(N) + 2 * (size_t)kMlpParams)))
+        return SBB_ERR_NOMEM;
+    float *parts = static_cast<float *>(mem.p);
+    float *mo = parts + mlp_parts_floats(N), *vo = mo + kMlpParams;
     SBB_CUDA(cudaMemsetAsync(mo, 0, sizeof(float) * 2 * kMlpParams, s));
-    for (int k = 1; k <= steps; k++) {
-        launch_mlp_forward(d_params, d_x, N, a.xn, a.h1, a.h2, a.y, s);
-        launch_mlp_backward(d_params, N, a.xn, a.h1, a.h2, a.y, d_t, d_w, inv, a.dy, a.dz2,
-                            a.dz1, g, d_loss_hist ? d_loss_hist + (k - 1) : nullptr, s);
-        launch_mlp_adam(d_params, g, mo, vo, k, lr, wd, s);
-    }
+    for (int k = 1; k <= steps; k++)
+        launch_mlp_step(d_params, d_x, N, d_t, d_w, inv, parts, mo, vo, k, lr, wd,
+                        d_loss_hist ? d_loss_hist + (k - 1) : nullptr, s);
     SBB_CUDA(cudaGetLastError());
     return SBB_OK;
 }
@@ -175,7 +148,7 @@ int sbb_mlp_select(const float *d_params, int m, int n, int nnz, const int *d_ro
     float *y = feat + kMlpFeatures;
     int *dcls = reinterpret_cast<int *>(y + 16);
     launch_features(d_rowptr, d_col, m, n, nnz, acc, feat, s);
-    launch_mlp_forward(d_params, feat, 1, nullptr, nullptr, nullptr, y, s);
+    launch_mlp_forward(d_params, feat, 1, y, s);
     launch_mlp_argmin(y, 1, dcls, s);
     SBB_CUDA(cudaMemcpyAsync(cls, dcls, sizeof(int), cudaMemcpyDeviceToHost, s));
     SBB_CUDA(cudaStreamSynchronize(s));

@@ -238,14 +238,16 @@ constexpr int kMlpParams = 2 * kMlpFeatures + kMlpHidden * kMlpFeatures + kMlpHi
 // acc: 8 device words of scratch; feat: 12 floats (device).
 void launch_features(const int *rp, const int *col, int m, int n, long long nnz,
                      unsigned long long *acc, float *feat, cudaStream_t s);
-void launch_mlp_forward(const float *P, const float *X, int N, float *Xn, float *H1, float *H2,
-                        float *Y, cudaStream_t s);
-void launch_mlp_backward(const float *P, int N, const float *Xn, const float *H1,
-                         const float *H2, const float *Y, const float *T, const float *W,
-                         float inv_norm, float *dY, float *dZ2, float *dZ1, float *G,
-                         float *loss, cudaStream_t s);
-void launch_mlp_adam(float *P, const float *G, float *M, float *V, int step, float lr, float wd,
-                     cudaStream_t s);
+void launch_mlp_forward(const float *P, const float *X, int N, float *Y, cudaStream_t s);
+// Gradient and loss (may be null) over N samples; `parts`: mlp_parts_floats(N)
+// floats of scratch.
+size_t mlp_parts_floats(int N);
+void launch_mlp_grad(const float *P, const float *X, int N, const float *T, const float *W,
+                     float inv_norm, float *parts, float *G, float *loss, cudaStream_t s);
+// The same followed by the Adam step number `step` on P, M, V.
+void launch_mlp_step(float *P, const float *X, int N, const float *T, const float *W,
+                     float inv_norm, float *parts, float *M, float *V, int step, float lr, float wd,
+                     float *loss, cudaStream_t s);
 void launch_mlp_argmin(const float *Y, int N, int *cls, cudaStream_t s);
 
 // Boundary pieces (drop-in): sum of val*x over [lo, hi) per piece.
