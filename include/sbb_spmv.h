@@ -129,7 +129,9 @@ typedef struct {
  * (int32 row pointer with rowptr[0] == 0 and rowptr[m] == nnz, int32 columns,
  * FP64 values).  The arrays must stay valid and unchanged while the plan
  * lives.  cfg may be NULL (automatic choice).  stream: a cudaStream_t or
- * NULL.  The row pointer is validated (one synchronisation). */
+ * NULL.  The row pointer is validated (one synchronisation).  Plans and
+ * host-pointer calls take device memory from a pool of the library's own,
+ * which keeps at most 1/32 of the device's memory between calls. */
 int sbb_plan_create(sbb_plan_t *plan, int m, int n, int nnz,
                     const int *d_rowptr, const int *d_col, const double *d_val,
                     const sbb_config *cfg, void *stream);

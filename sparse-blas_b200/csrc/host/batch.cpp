@@ -40,6 +40,7 @@ struct sbb_batch_s {
 
 static void batch_free(sbb_batch_s *b)
 {
+    cudaDeviceSynchronize();  // products in flight on any stream
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     if (b->cap) cudaStreamDestroy(b->cap);
@@ -58,7 +59,7 @@ static void batch_free(sbb_batch_s *b)
         if (b->d_unit0[f]) cudaFree(b->d_unit0[f]);
     }
     for (Plan *p : b->plans) {
-        plan_free(p);
+        plan_free(p, nullptr);
         delete p;
     }
     delete b;
@@ -418,7 +419,6 @@ int sbb_batch_destroy(sbb_batch_t b)
 {
     if (!b) return SBB_OK;
     cudaSetDevice(b->device);
-    cudaDeviceSynchronize();
     batch_free(b);
     return SBB_OK;
 }
@@ -456,8 +456,7 @@ int sbb_tune_classes(int m, int n, int nnz, const int *d_rowptr, const int *d_co
             cudaEventElapsedTime(&t, e0, e1);
             ms[cls] = t / reps;
         }
-        cudaStreamSynchronize(s);
-        plan_free(&p);
+        plan_free(&p, s);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

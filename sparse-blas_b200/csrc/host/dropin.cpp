@@ -31,7 +31,6 @@
 namespace sbb {
 
 int plan_build_unchecked(Plan *p, const sbb_config *cfg, cudaStream_t s);
-void plan_free_async(Plan *p, cudaStream_t s);
 
 // Same bisection as src/spmv_helper.cu:16-39 (the partition must match the
 // reference exactly, including which row of a run of empty rows it returns).
@@ -151,7 +150,6 @@ void trace_mark(int k)
 
 struct ThreadState {
     cudaStream_t s[2][64] = {};
-    bool pool_set[64] = {};
     unsigned *words = nullptr;
     ~ThreadState()
     {
@@ -167,20 +165,11 @@ ThreadState &thread_state()
     return t;
 }
 
-// Per-thread stream; device memory comes from the device's default pool,
-// which keeps freed blocks for the next call.
+// Per-thread stream.
 cudaStream_t call_stream(int dev, int which = 0)
 {
     ThreadState &t = thread_state();
     if (dev < 0 || dev >= 64) return 0;
-    if (!t.pool_set[dev]) {
-        cudaMemPool_t pool;
-        if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-            unsigned long long keep = ~0ull;
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        }
-        t.pool_set[dev] = true;
-    }
     if (!t.s[which][dev] &&
         cudaStreamCreateWithFlags(&t.s[which][dev], cudaStreamNonBlocking) != cudaSuccess)
         t.s[which][dev] = nullptr;
@@ -286,7 +275,12 @@ int run(int m, int n, long long nnz, double alpha, const double *val, const long
     const int hm = hr1 - hr0 + 1;
     double need = (double)nnz * 12.0 + ((double)m + 1.0) * 12.0 + (double)n * 8.0 + (double)hm * 8.0 +
                   (double)((long long)hm + nnz) / 256.0 * 24.0;
-    if (need / 1e9 > 0.8 * ((double)free_b / 1e9)) return -1;
+    if (need / 1e9 > 0.8 * ((double)free_b / 1e9)) {
+        pool_trim();  // memory the pool keeps counts as used until it is given back
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return -1;
+        free_b = capped_free_bytes(free_b);
+        if (need / 1e9 > 0.8 * ((double)free_b / 1e9)) return -1;
+    }
 
     int dev = 0;
     cudaGetDevice(&dev);
@@ -409,7 +403,7 @@ int run(int m, int n, long long nnz, double alpha, const double *val, const long
     if (rc != SBB_OK) {
         cudaStreamSynchronize(s2);
         cudaStreamSynchronize(s);
-        for (auto &p : plans) plan_free_async(&p, s2);
+        for (auto &p : plans) plan_free(&p, s2);
         cudaStreamSynchronize(s2);
         destroy_events();
         return rc == SBB_ERR_NOMEM ? 1 : -1;
@@ -428,7 +422,7 @@ int run(int m, int n, long long nnz, double alpha, const double *val, const long
         double *d_ps = B.get<double>(pieces.size());
         if (!B.ok) {
             cudaStreamSynchronize(s2);
-            for (auto &p : plans) plan_free_async(&p, s2);
+            for (auto &p : plans) plan_free(&p, s2);
             cudaStreamSynchronize(s2);
             destroy_events();
             return 1;
@@ -450,7 +444,7 @@ int run(int m, int n, long long nnz, double alpha, const double *val, const long
     ck(cudaStreamSynchronize(s));
     trace_mark(4);
     ck(cudaGetLastError());
-    for (auto &p : plans) plan_free_async(&p, s);
+    for (auto &p : plans) plan_free(&p, s);
     destroy_events();
     if (!cuda_ok) return -1;
     // Restore the rows the reference never writes, and the special rows'

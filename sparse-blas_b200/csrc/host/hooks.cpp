@@ -28,7 +28,7 @@ cudaError_t dev_malloc_async(void **p, size_t bytes, cudaStream_t s)
         *p = nullptr;
         return cudaErrorMemoryAllocation;
     }
-    return cudaMallocAsync(p, bytes, s);
+    return pool_malloc_async(p, bytes, s);
 }
 
 size_t capped_free_bytes(size_t free_b)

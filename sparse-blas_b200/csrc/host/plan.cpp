@@ -128,36 +128,19 @@ static int dalloc(T **p, size_t count, cudaStream_t s, size_t *acc)
     return SBB_OK;
 }
 
-extern void sliced_free_async(Plan *, cudaStream_t);
+extern void tiled_free(Plan *, cudaStream_t);
+extern void rows_free(Plan *, cudaStream_t);
+extern void sliced_free(Plan *, cudaStream_t);
 
-void plan_free_async(Plan *p, cudaStream_t s)
+void plan_free(Plan *p, cudaStream_t s)
 {
     void *ptrs[] = {p->tile_row, p->tile_nnz, p->carry_val, p->queue, p->status};
     for (void *q : ptrs)
         if (q) cudaFreeAsync(q, s);
-    carry_runs_free(&p->runs, s, true);
-    extern void tiled_free_async(Plan *, cudaStream_t);
-    tiled_free_async(p, s);
-    extern void rows_free_async(Plan *, cudaStream_t);
-    rows_free_async(p, s);
-    sliced_free_async(p, s);
-    p->tile_row = p->tile_nnz = nullptr;
-    p->carry_val = nullptr;
-    p->queue = p->status = nullptr;
-}
-
-void plan_free(Plan *p)
-{
-    void *ptrs[] = {p->tile_row, p->tile_nnz, p->carry_val, p->queue, p->status};
-    for (void *q : ptrs)
-        if (q) cudaFree(q);
-    carry_runs_free(&p->runs, 0, false);
-    extern void tiled_free(Plan *);
-    tiled_free(p);
-    extern void rows_free(Plan *);
-    rows_free(p);
-    extern void sliced_free(Plan *);
-    sliced_free(p);
+    carry_runs_free(&p->runs, s);
+    tiled_free(p, s);
+    rows_free(p, s);
+    sliced_free(p, s);
     p->tile_row = p->tile_nnz = nullptr;
     p->carry_val = nullptr;
     p->queue = p->status = nullptr;
@@ -203,7 +186,7 @@ static int build_sliced(Plan *p, int width, bool fall_back, cudaStream_t s)
         rc = SBB_ERR_INPUT;
     }
     if (!fall_back || rc == SBB_ERR_CUDA) return rc;
-    sliced_free_async(p, s);
+    sliced_free(p, s);
     p->vector_width = vw;
     p->scratch_bytes = bytes;
     SBB_CUDA(cudaMemsetAsync(p->status, 0, 4 * sizeof(unsigned), s));
@@ -475,8 +458,8 @@ static int create_common(sbb_plan_t *out, int m, int n, int nnz, const int *rp, 
     h->p.lane32 = lane32;
     int rc = plan_build(&h->p, cfg, static_cast<cudaStream_t>(stream));
     if (rc != SBB_OK) {
+        plan_free(&h->p, static_cast<cudaStream_t>(stream));
         cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
-        plan_free(&h->p);
         delete h;
         return rc;
     }
@@ -616,8 +599,8 @@ int sbb_plan_destroy(sbb_plan_t plan)
 {
     if (!plan) return SBB_OK;
     cudaSetDevice(plan->p.device);
-    cudaDeviceSynchronize();
-    plan_free(&plan->p);
+    cudaDeviceSynchronize();  // products in flight on any stream
+    plan_free(&plan->p, nullptr);
     delete plan;
     return SBB_OK;
 }

@@ -189,15 +189,10 @@ int carry_runs_build_device(const int *crow, int T, int m, CarryRuns *R, cudaStr
     return SBB_OK;
 }
 
-void carry_runs_free(CarryRuns *R, cudaStream_t s, bool async)
+void carry_runs_free(CarryRuns *R, cudaStream_t s)
 {
     for (int *p : {R->run_first, R->run_len, R->count})
-        if (p) {
-            if (async)
-                cudaFreeAsync(p, s);
-            else
-                cudaFree(p);
-        }
+        if (p) cudaFreeAsync(p, s);
     R->count = nullptr;
     R->run_first = R->run_len = nullptr;
     R->n_runs = 0;

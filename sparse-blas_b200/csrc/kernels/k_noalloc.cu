@@ -24,8 +24,6 @@
 //     capture on that device.  The address is kept per device together with
 //     the identity of the context it was found in, and looked up again when
 //     that context has been replaced (after cudaDeviceReset, for example).
-#include <cuda.h>  // driver types only; the entry points are fetched at run time
-
 #include <mutex>
 
 #include "../sbb_internal.h"
@@ -55,35 +53,6 @@ struct ScratchAddr {
     unsigned long long ctx = 0;  // identity of the context the address belongs to
 };
 ScratchAddr g_scratch_addr[64];
-
-// Unique id of the calling thread's current context, or 0 when there is none
-// or the driver cannot tell (cuCtxGetId, CUDA 12.0+).  The driver entry
-// points are fetched through the runtime, so the library does not link
-// libcuda itself.
-unsigned long long current_context_id()
-{
-    using GetCurrent = CUresult (*)(CUcontext *);
-    using GetId = CUresult (*)(CUcontext, unsigned long long *);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        cudaDriverEntryPointQueryResult q;
-        void *f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(f);
-    });
-    if (!get_current || !get_id) return 0;
-    CUcontext c = nullptr;
-    if (get_current(&c) != CUDA_SUCCESS || !c) return 0;
-    unsigned long long id = 0;
-    return get_id(c, &id) == CUDA_SUCCESS ? id : 0;
-}
 
 // Device address of the scratch on device `dev` (the current device): looked
 // up with that device current the first time, and again whenever the

@@ -530,25 +530,17 @@ int rows_run(Plan *p, double alpha, const void *x, double beta, double *y, cudaS
     return SBB_OK;
 }
 
-static void rows_release(Plan *p, cudaStream_t s, bool async)
+void rows_free(Plan *p, cudaStream_t s)
 {
     auto *R = static_cast<RowsPlan *>(p->rows);
     if (!R) return;
     void *ptrs[] = {R->desc, R->carry_row, R->carry_val};
     for (void *q : ptrs)
-        if (q) {
-            if (async)
-                cudaFreeAsync(q, s);
-            else
-                cudaFree(q);
-        }
-    carry_runs_free(&R->runs, s, async);
+        if (q) cudaFreeAsync(q, s);
+    carry_runs_free(&R->runs, s);
     delete R;
     p->rows = nullptr;
 }
-
-void rows_free(Plan *p) { rows_release(p, 0, false); }
-void rows_free_async(Plan *p, cudaStream_t s) { rows_release(p, s, true); }
 
 int rows_launches(const Plan *p)
 {

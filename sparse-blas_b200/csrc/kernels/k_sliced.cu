@@ -271,23 +271,15 @@ int sliced_run(Plan *p, double alpha, const void *x, double beta, double *y, cud
     return SBB_OK;
 }
 
-static void sliced_release(Plan *p, cudaStream_t s, bool async)
+void sliced_free(Plan *p, cudaStream_t s)
 {
     auto *S = static_cast<SlicedPlan *>(p->sliced);
     if (!S) return;
     void *ptrs[] = {S->col, S->val};
     for (void *q : ptrs)
-        if (q) {
-            if (async)
-                cudaFreeAsync(q, s);
-            else
-                cudaFree(q);
-        }
+        if (q) cudaFreeAsync(q, s);
     delete S;
     p->sliced = nullptr;
 }
-
-void sliced_free(Plan *p) { sliced_release(p, 0, false); }
-void sliced_free_async(Plan *p, cudaStream_t s) { sliced_release(p, s, true); }
 
 }  // namespace sbb

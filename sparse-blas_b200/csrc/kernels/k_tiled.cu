@@ -579,25 +579,17 @@ int tiled_run(Plan *p, double alpha, const void *x, double beta, double *y, cuda
     return SBB_OK;
 }
 
-static void tiled_release(Plan *p, cudaStream_t s, bool async)
+void tiled_free(Plan *p, cudaStream_t s)
 {
     auto *T = static_cast<TiledPlan *>(p->tiled);
     if (!T) return;
     void *ptrs[] = {T->blob, T->tile_seg, T->ne, T->empty, T->carry_row, T->carry_val};
     for (void *q : ptrs)
-        if (q) {
-            if (async)
-                cudaFreeAsync(q, s);
-            else
-                cudaFree(q);
-        }
-    carry_runs_free(&T->runs, s, async);
+        if (q) cudaFreeAsync(q, s);
+    carry_runs_free(&T->runs, s);
     delete T;
     p->tiled = nullptr;
 }
-
-void tiled_free(Plan *p) { tiled_release(p, 0, false); }
-void tiled_free_async(Plan *p, cudaStream_t s) { tiled_release(p, s, true); }
 
 int tiled_launches(const Plan *p)
 {

@@ -32,8 +32,19 @@ inline bool ranges_overlap(const void *a, size_t abytes, const void *b, size_t b
     return pa < pb + bbytes && pb < pa + abytes;
 }
 
+// ---- device memory (pool.cpp) ----------------------------------------------
+// Stream-ordered memory from the library's pool on the current device; freed
+// with cudaFreeAsync.
+cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
+// Gives the pool's unused memory back to the system.
+void pool_trim();
+// Unique id of the calling thread's current context, or 0 when there is none
+// or the driver cannot tell (cuCtxGetId, CUDA 12.0+).  The driver entry points
+// are fetched through the runtime, so the library does not link libcuda itself.
+unsigned long long current_context_id();
+
 // ---- test hooks (hooks.cpp; armed only by sbb_test_hook) -------------------
-// cudaMallocAsync, except that an armed allocation-failure hook fails it.
+// pool_malloc_async, except that an armed allocation-failure hook fails it.
 cudaError_t dev_malloc_async(void **p, size_t bytes, cudaStream_t s);
 // Free device memory as the drop-in memory pre-check sees it.
 size_t capped_free_bytes(size_t free_b);
@@ -125,7 +136,7 @@ int carry_runs_build(const int *carry_row, int T, int m, CarryRuns *R, cudaStrea
 // The same lists built without any host synchronisation: runs in the order
 // the marking kernel found them, their count left on the device (R->count).
 int carry_runs_build_device(const int *carry_row, int T, int m, CarryRuns *R, cudaStream_t s);
-void carry_runs_free(CarryRuns *R, cudaStream_t s, bool async);
+void carry_runs_free(CarryRuns *R, cudaStream_t s);
 // Marks the runs on the device only; the count stays in *dev_count.
 void launch_runs_mark(const int *carry_row, int T, int m, int *run_first, int *run_len,
                       int *dev_count, cudaStream_t s);
@@ -288,7 +299,8 @@ struct Plan {
 int plan_build(Plan *p, const sbb_config *cfg, cudaStream_t s);
 int plan_run(Plan *p, double alpha, const void *x, double beta, double *y,
              cudaStream_t s);
-void plan_free(Plan *p);
+// Frees the plan's device memory in stream order on s.
+void plan_free(Plan *p, cudaStream_t s);
 int default_kernel_choice(int m, int nnz, int max_row, int *vector_width, int *ipt, int *sigma);
 int plan_launches(const Plan *p);
 // Optional timing hooks (set by sbb_spmv_timed for the calling thread): the
