@@ -37,6 +37,8 @@ __device__ __forceinline__ float4 ld_stream(const float4 *p) { return __ldcs(p);
 SBB_LOAD_IF(ld_stream_if, int, "r", "b32", "ld.global.cs")
 SBB_LOAD_IF(ld_stream_if, float, "f", "b32", "ld.global.cs")
 SBB_LOAD_IF(ld_stream_if, double, "d", "b64", "ld.global.cs")
+SBB_LOAD_IF(ld_x_if, float, "f", "b32", "ld.global.nc")
+SBB_LOAD_IF(ld_x_if, double, "d", "b64", "ld.global.nc")
 SBB_KEEP_IF(float, "f", "b32")
 SBB_KEEP_IF(double, "d", "b64")
 #undef SBB_LOAD_IF
@@ -92,6 +94,14 @@ __device__ __forceinline__ T gather_x(const T *x, int c, int n, unsigned &bad)
     if ((unsigned)c < (unsigned)n) return ld_x(x + c);
     bad = 1u;
     return T(0);
+}
+
+template <typename T>
+__device__ __forceinline__ T gather_x_if(const T *x, int c, int n, bool p, unsigned &bad)
+{
+    const bool ok = (unsigned)c < (unsigned)n;
+    bad |= p && !ok;
+    return ld_x_if(x + c, p && ok);
 }
 
 // Per-value products for the two storage forms.
@@ -168,6 +178,15 @@ __device__ __forceinline__ void write_y(double *yp, double alpha, double sum, do
                                         uint64_t pol)
 {
     st_y(yp, y_update(alpha, sum, beta, beta == 0.0 ? 0.0 : ld_y(yp, pol)), pol);
+}
+
+// Starts bringing [a, a + bytes) into L2 (whole 16-byte pieces around it: the
+// array must be 16-byte aligned and its allocation end on such a boundary).
+__device__ __forceinline__ void prefetch_l2(const void *a, size_t bytes)
+{
+    const uint64_t lo = reinterpret_cast<uint64_t>(a) & ~15ull;
+    const uint32_t n = (uint32_t)((reinterpret_cast<uint64_t>(a) + bytes + 15 - lo) & ~15ull);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"(n) : "memory");
 }
 
 // Programmatic dependent launch (sm_90+): a kernel launched with the

@@ -15,10 +15,10 @@
 // most of them in the butterflies and the ragged ends of each row) and
 // latency come before HBM (24 %).  Here a step of 32 nnz takes about 16
 // instructions.  Measured against it (FP64, beta = 0.5; us): 200k rows of 24
-// nnz in a band 14.4 vs 26.7; 500k rows of 6 11.8 vs 19.1; 100k rows of 50 in
-// diagonal blocks 15.0 vs 21.5; 1M rows of 40 in a band 91.6 vs 136.5 (5.5 TB/s);
+// nnz in a band 13.6 vs 26.7; 500k rows of 6 10.6 vs 19.1; 100k rows of 50 in
+// diagonal blocks 14.4 vs 21.5; 1M rows of 40 in a band 91.6 vs 136.5 (5.5 TB/s);
 // 700k rows of 0 to 8, half of them empty, 12.0 vs 16.3; FP32 storage, 200k
-// rows of 24, 13.5 vs 24.3.  What bounds it now: HBM on the largest of these,
+// rows of 24, 12.7 vs 24.3.  What bounds it now: HBM on the largest of these,
 // on the others the chain of row pointer, column and x loads of each slice and
 // one to three waves of warps.
 #include <stdint.h>
@@ -38,6 +38,13 @@ constexpr int ST = 256;  // threads per CTA
 // with no bound the compiler unrolls the step loops to 148 registers, 53 us.
 constexpr int kSteps = 4;
 constexpr int kMinCtas = 6;
+// Slices of up to this many nnz in the mean are brought into L2 as a whole
+// when their place is known, so that HBM's latency is paid once and not every
+// kSteps steps (us, without and with: 100k rows of 12 7.1 and 5.9, 500k of 6
+// 11.8 and 10.6, 200k of 24 14.4 and 13.6, 100k of 50 14.9 and 14.4); in longer
+// ones the loads in flight are enough and the prefetches only crowd L2 (rows of
+// 100, 800 nnz a slice: 26.4 and 32.7; of 40, 640 nnz: 91.9 and 97.3).
+constexpr int kPrefetchNnz = 448;
 
 struct SlicedPlan {
     int width = 1;  // lanes per row
@@ -45,11 +52,12 @@ struct SlicedPlan {
     void *val = nullptr;
 };
 
-// What a lane knows of its slice: its row (sub-lane 0 writes it), how many nnz
-// it takes, the steps of the slice and those that every lane takes part in.
+// What a lane knows of its slice: its row (-1: none; sub-lane 0 writes it), the
+// slice's first nnz and their number, how many nnz the lane takes, the steps of
+// the slice and those that every lane takes part in.
 struct SliceLane {
     int row;
-    unsigned base;  // first nnz of the slice
+    unsigned base, total;
     int start, len, mine, steps, full;
 };
 template <int W>
@@ -69,13 +77,14 @@ __device__ __forceinline__ SliceLane slice_lane(int s, int m, const int *__restr
         L.row = -1;
     }
     L.base = (unsigned)__shfl_sync(0xffffffffu, L.start, 0);
+    L.total = __reduce_add_sync(0xffffffffu, sub == 0 ? (unsigned)L.len : 0u);
     L.mine = L.len > sub ? (L.len - sub + W - 1) / W : 0;
     L.steps = __reduce_max_sync(0xffffffffu, L.mine);
     L.full = __reduce_min_sync(0xffffffffu, L.mine);
     return L;
 }
 
-template <typename PT, typename ACC, int W>
+template <typename PT, typename ACC, int W, bool PREFETCH>
 __global__ void __launch_bounds__(ST, kMinCtas)
 sliced_kernel(int m, int slices, const int *__restrict__ rowptr, const int *__restrict__ col,
               const typename PT::V *__restrict__ val, const typename PT::V *__restrict__ x,
@@ -87,6 +96,10 @@ sliced_kernel(int m, int slices, const int *__restrict__ rowptr, const int *__re
     const int lane = threadIdx.x & 31;
     const uint64_t keep = l2_evict_last(), stream = l2_evict_first();
     const SliceLane L = slice_lane<W>(s, m, rowptr);
+    if (PREFETCH && L.steps > kSteps && lane == 0) {
+        prefetch_l2(col + L.base, 4 * (size_t)L.total);
+        prefetch_l2(val + L.base, sizeof(V) * (size_t)L.total);
+    }
     const bool writes = L.row >= 0 && lane % W == 0;
     double yv = 0.0;
     if (writes && beta != 0.0) yv = ld_y(y + L.row, stream);
@@ -158,8 +171,7 @@ slice_fill_kernel(const int *__restrict__ rowptr, int m, int n, int slices,
     const int s = (int)((long long)blockIdx.x * kFillWarps + warp);
     if (s >= slices) return;  // no block-wide barrier follows
     const SliceLane L = slice_lane<W>(s, m, rowptr);
-    const unsigned total =
-        __reduce_add_sync(0xffffffffu, lane % W == 0 ? (unsigned)L.len : 0u);
+    const unsigned total = L.total;
     const bool staged = total <= kFillNnz;
     bool bad = false;
     if (staged) {
@@ -213,8 +225,11 @@ void run_w(const SlicedPlan &S, const Plan *p, double alpha, const void *x, doub
 {
     using V = typename PT::V;
     const int slices = slices_of<W>(p->m);
+    const auto kern = (long long)p->nnz <= (long long)kPrefetchNnz * slices
+                          ? sliced_kernel<PT, ACC, W, true>
+                          : sliced_kernel<PT, ACC, W, false>;
     hook_start(s);
-    sliced_kernel<PT, ACC, W><<<(int)(((long long)slices * 32 + ST - 1) / ST), ST, 0, s>>>(
+    kern<<<(int)(((long long)slices * 32 + ST - 1) / ST), ST, 0, s>>>(
         p->m, slices, p->rowptr, S.col, static_cast<const V *>(S.val), static_cast<const V *>(x), y,
         alpha, beta);
     hook_stop(s);
@@ -242,7 +257,9 @@ int sliced_build(Plan *p, cudaStream_t s)
         p->scratch_bytes += bytes;
         return dev_malloc_async(ptr, bytes, s) == cudaSuccess;
     };
-    if (!al((void **)&S->col, sizeof(int) * (size_t)p->nnz) || !al(&S->val, vb * (size_t)p->nnz)) {
+    // 16 bytes more than the nnz: prefetches run to the next 16-byte boundary
+    if (!al((void **)&S->col, sizeof(int) * (size_t)p->nnz + 16) ||
+        !al(&S->val, vb * (size_t)p->nnz + 16)) {
         set_error("sliced plan: device allocation failed");
         return SBB_ERR_NOMEM;
     }
