@@ -20,9 +20,9 @@ struct sbb_batch_s {
     long long *d_unit0[kBatchFamilies] = {};
     int fcount[kBatchFamilies] = {};
     long long total[kBatchFamilies] = {};
-    int grid[kBatchFamilies] = {};
+    int grid[kBatchFamilies] = {}, claim[kBatchFamilies] = {};
     double fbytes[kBatchFamilies] = {};
-    unsigned long long *d_queue = nullptr;  // [f]: family f's next claim of kBatchClaim units
+    unsigned long long *d_queue = nullptr;  // [f]: family f's next claim
     unsigned *d_status = nullptr;
     cudaStream_t side[kBatchFamilies - 1] = {};  // branches for the other families
     cudaEvent_t ev_fork = nullptr, ev_join[kBatchFamilies - 1] = {};
@@ -87,8 +87,8 @@ static int enqueue(sbb_batch_s *b, cudaStream_t s)
         const int f = fams[j];
         cudaStream_t st = j == 0 ? s : b->side[j - 1];
         if (j > 0) SBB_CUDA(cudaStreamWaitEvent(st, b->ev_fork, 0));
-        launch_batch(f, b->d_fmats[f], b->fcount[f], b->d_unit0[f], b->total[f], b->d_queue + f,
-                     b->d_status, b->grid[f], st);
+        launch_batch(f, b->d_fmats[f], b->fcount[f], b->d_unit0[f], b->total[f], b->claim[f],
+                     b->d_queue + f, b->d_status, b->grid[f], st);
         if (j > 0) SBB_CUDA(cudaEventRecord(b->ev_join[j - 1], st));
     }
     for (size_t j = 1; j < fams.size(); j++) SBB_CUDA(cudaStreamWaitEvent(s, b->ev_join[j - 1], 0));
@@ -247,7 +247,7 @@ int sbb_batch_create(sbb_batch_t *out, const sbb_batch_item *items, int count, v
             }
         } else {
             // units of about kBatchVectorNnz nnz: vsteps chunks of cr rows
-            const long long cr = vector_chunk_rows(4 << it.cls, kBatchVectorU);
+            const long long cr = vector_chunk(4 << it.cls);
             const double mean = it.m > 0 ? (double)it.nnz / it.m : 1.0;
             long long steps = (long long)(kBatchVectorNnz / (cr * std::max(mean, 1.0)) + 0.5);
             steps = std::min<long long>(64, std::max<long long>(1, steps));
@@ -337,8 +337,16 @@ int sbb_batch_create(sbb_batch_t *out, const sbb_batch_item *items, int count, v
     b->fix_slots = tile0.back();
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-    for (int f = 0; f < kBatchFamilies; f++)
+    for (int f = 0; f < kBatchFamilies; f++) {
         b->grid[f] = sms * std::max(batch_max_ctas_per_sm(f), 1);
+        // The grid's warps claim at least eight times each in the mean, so the
+        // last claims are a small part of the whole.  With 16 units of 1,024
+        // nnz in every claim most warps had none or one: 30 matrices of up to
+        // 8,000 rows took 875 us, 64 of up to 200,000 930 us; now 38 and 362.
+        const long long warps = (long long)b->grid[f] * 8;
+        b->claim[f] =
+            (int)std::min<long long>(kBatchClaim, std::max<long long>(1, b->total[f] / (8 * warps)));
+    }
     *out = b;
     return SBB_OK;
 }

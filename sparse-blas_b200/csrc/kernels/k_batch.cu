@@ -6,7 +6,7 @@
 // tiled class) has one persistent kernel and one device work queue: every
 // matrix of the family contributes work units - row chunks, warp segments or
 // groups of kBatchTileGroup tiles - and the warps of the family's grid claim
-// kBatchClaim consecutive units per queue access (one atomic on one counter)
+// a number of consecutive units per queue access (one atomic on one counter)
 // until the queue is empty.  The families' kernels run side by side (parallel
 // branches of one stream or graph); a kernel holds only its family's code, so
 // it gets the register budget and occupancy that code needs.  A unit runs
@@ -36,10 +36,8 @@ static_assert(TBB % 16 == 0, "bulk copies move multiples of 16 bytes");
 
 // Per class kernel: dynamic shared memory per warp (merge: a segment's
 // staging; tiled: two unit slots) and the CTAs per SM its register budget
-// aims at.  The vector families spill a few dozen bytes at 64 registers;
-// at 3 CTAs per SM they do not, but the 512-matrix batch ran slower (4.85
-// vs 4.73 ms).
-template <int FAM> struct FamShape {  // vector families
+// aims at.
+template <int FAM> struct FamShape {  // vector classes
     static constexpr size_t kWarpBytes = 0;
     static constexpr int MINB = 4;
 };
@@ -60,20 +58,15 @@ template <int FAM> __device__ __forceinline__ unsigned char *warp_smem()
     return s_dyn + (size_t)(threadIdx.x >> 5) * FamShape<FAM>::kWarpBytes;
 }
 
-// A vector-class unit: vsteps consecutive chunks of CR rows (kBatchVectorU
-// rows of each lane group in flight: the batch kernel's register budget).
+// A vector-class unit: vsteps consecutive chunks of rows.
 template <int V>
 __device__ __forceinline__ void vector_unit(const BatchMat &M, int local, unsigned &bad)
 {
-    constexpr int U = kBatchVectorU;
-    constexpr int CR = VectorShape<V, U>::CR;
-    static_assert(CR == vector_chunk_rows(V, U), "host and device chunk sizes differ");
-    const uint64_t stream = l2_evict_first();
-    const long long r0 = (long long)local * CR * M.vsteps;
-    for (int s = 0; s < M.vsteps && r0 + (long long)CR * s < M.m; ++s)
-        vector_chunk<ProdF64, AccF64, V, U>((int)(r0 + (long long)CR * s), M.m, M.n, M.rowptr,
-                                            M.col, static_cast<const double *>(M.val), M.x, M.y,
-                                            M.alpha, M.beta, stream, bad);
+    const int share = vector_chunk(V) * M.vsteps;
+    const long long r0 = (long long)local * share;
+    vector_rows<ProdF64, AccF64, V>((int)r0, (int)min((long long)share, M.m - r0), M.n, M.rowptr,
+                                    M.col, static_cast<const double *>(M.val), M.x, M.y, M.alpha,
+                                    M.beta, l2_evict_first(), bad);
 }
 
 __device__ __forceinline__ int find_matrix(const long long *unit0, int nmat, long long u)
@@ -104,7 +97,7 @@ __device__ __forceinline__ ClaimSpan claim_span(const long long *unit0, int i, l
 template <int FAM>
 __global__ void __launch_bounds__(BT, FamShape<FAM>::MINB)
 batch_kernel(const BatchMat *__restrict__ mats, int nmat, const long long *__restrict__ unit0,
-             long long total, unsigned long long *queue, unsigned *status)
+             long long total, int claim, unsigned long long *queue, unsigned *status)
 {
     constexpr bool kTiled = FAM == kFamTiled;
     __shared__ __align__(8) uint64_t bars[kTiled ? BW : 1][2];
@@ -138,9 +131,9 @@ batch_kernel(const BatchMat *__restrict__ mats, int nmat, const long long *__res
         unsigned long long c = 0;
         if (lane == 0) c = atomicAdd(queue, 1ull);
         c = __shfl_sync(0xffffffffu, c, 0);
-        const long long u0 = (long long)c * kBatchClaim;
+        const long long u0 = (long long)c * claim;
         if (u0 >= total) break;
-        const int n = (int)(total - u0 < kBatchClaim ? total - u0 : kBatchClaim);
+        const int n = (int)(total - u0 < claim ? total - u0 : claim);
         int i = find_matrix(unit0, nmat, u0);
         ClaimSpan sp = claim_span(unit0, i, u0, n);
         for (int k = 0; k < n; ++k) {
@@ -150,16 +143,13 @@ batch_kernel(const BatchMat *__restrict__ mats, int nmat, const long long *__res
             }
             const BatchMat &M = mats[i];
             const int local = k - sp.first;
-            if constexpr (FAM == kFamVectorNarrow) {
-                if (M.cls == 0)
-                    vector_unit<4>(M, local, bad);
-                else
-                    vector_unit<8>(M, local, bad);
-            } else if constexpr (FAM == kFamVectorWide) {
-                if (M.cls == 2)
-                    vector_unit<16>(M, local, bad);
-                else
-                    vector_unit<32>(M, local, bad);
+            if constexpr (FAM == kFamVector) {
+                switch (M.cls) {
+                case 0: vector_unit<4>(M, local, bad); break;
+                case 1: vector_unit<8>(M, local, bad); break;
+                case 2: vector_unit<16>(M, local, bad); break;
+                default: vector_unit<32>(M, local, bad); break;
+                }
             } else if constexpr (FAM == kFamMerge) {
                 unsigned char *wsm = warp_smem<FAM>();
                 merge_segment<ProdF64, AccF64, kBatchIpt>(
@@ -292,30 +282,30 @@ template <int FAM> static int max_ctas()
 int batch_max_ctas_per_sm(int fam)
 {
     switch (fam) {
-    case 0: return max_ctas<0>();
-    case 1: return max_ctas<1>();
-    case 2: return max_ctas<2>();
-    default: return max_ctas<3>();
+    case kFamVector: return max_ctas<kFamVector>();
+    case kFamMerge: return max_ctas<kFamMerge>();
+    default: return max_ctas<kFamTiled>();
     }
 }
 
 template <int FAM>
 static void launch_fam(const BatchMat *mats, int nmat, const long long *unit0, long long total,
-                       unsigned long long *queue, unsigned *status, int grid, cudaStream_t s)
+                       int claim, unsigned long long *queue, unsigned *status, int grid,
+                       cudaStream_t s)
 {
-    batch_kernel<FAM><<<grid, BT, fam_smem<FAM>(), s>>>(mats, nmat, unit0, total, queue, status);
+    batch_kernel<FAM><<<grid, BT, fam_smem<FAM>(), s>>>(mats, nmat, unit0, total, claim, queue,
+                                                        status);
 }
 
 void launch_batch(int fam, const BatchMat *mats, int nmat, const long long *unit0,
-                  long long total, unsigned long long *queue, unsigned *status, int grid,
-                  cudaStream_t s)
+                  long long total, int claim, unsigned long long *queue, unsigned *status,
+                  int grid, cudaStream_t s)
 {
     if (total <= 0 || nmat <= 0) return;
     switch (fam) {
-    case 0: launch_fam<0>(mats, nmat, unit0, total, queue, status, grid, s); break;
-    case 1: launch_fam<1>(mats, nmat, unit0, total, queue, status, grid, s); break;
-    case 2: launch_fam<2>(mats, nmat, unit0, total, queue, status, grid, s); break;
-    default: launch_fam<3>(mats, nmat, unit0, total, queue, status, grid, s); break;
+    case kFamVector: launch_fam<kFamVector>(mats, nmat, unit0, total, claim, queue, status, grid, s); break;
+    case kFamMerge: launch_fam<kFamMerge>(mats, nmat, unit0, total, claim, queue, status, grid, s); break;
+    default: launch_fam<kFamTiled>(mats, nmat, unit0, total, claim, queue, status, grid, s); break;
     }
 }
 

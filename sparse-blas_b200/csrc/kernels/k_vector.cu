@@ -6,8 +6,10 @@
 // coalesced streaming loads (V consecutive nnz per step), gathers x through
 // the read-only path and reduces with warp shuffles (xor butterfly: the order
 // is fixed for a given V), with several rows' loads in flight per group
-// (vector_chunk).  Good for regular matrices whose row lengths are close to
+// (vector_rows).  Good for regular matrices whose row lengths are close to
 // V; long rows serialise on one group.
+#include <algorithm>
+
 #include "../sbb_internal.h"
 #include "common.cuh"
 #include "spmv_device.cuh"
@@ -18,22 +20,38 @@ namespace {
 
 constexpr int VT = 256;  // threads per CTA
 
-// Warp w of the grid takes chunks w, w + W, ... of CR rows (W = all warps).
+// Warp w of the grid takes rows [w * share, (w + 1) * share).
 template <typename PT, typename ACC, int V>
-__global__ void __launch_bounds__(VT)
+__global__ void __launch_bounds__(VT, 4)
 vector_kernel(int m, int n, const int *__restrict__ rowptr, const int *__restrict__ col,
               const typename PT::V *__restrict__ val, const typename PT::V *__restrict__ x,
-              double *__restrict__ y, double alpha, double beta, unsigned *status)
+              double *__restrict__ y, double alpha, double beta, unsigned *status, int share)
 {
-    constexpr int CR = VectorShape<V>::CR;
-    static_assert(CR == vector_chunk_rows(V, V < 4 ? V : 4), "host and device chunk sizes differ");
-    const int warps = gridDim.x * (VT / 32);
-    const int chunks = (int)(((long long)m + CR - 1) / CR);
-    const uint64_t stream = l2_evict_first();
+    const long long r0 = ((long long)blockIdx.x * (VT / 32) + (threadIdx.x >> 5)) * share;
+    if (r0 >= m) return;
     unsigned bad = 0;
-    for (int c = blockIdx.x * (VT / 32) + (threadIdx.x >> 5); c < chunks; c += warps)
-        vector_chunk<PT, ACC, V>(c * CR, m, n, rowptr, col, val, x, y, alpha, beta, stream, bad);
+    vector_rows<PT, ACC, V>((int)r0, (int)min((long long)share, m - r0), n, rowptr, col, val, x, y,
+                            alpha, beta, l2_evict_first(), bad);
     if (bad) atomicOr(status, ST_BAD_COL);
+}
+
+template <typename PT, typename ACC, int V>
+void launch_vector_v(const CsrView &A, double alpha, const typename PT::V *x, double beta,
+                     double *y, unsigned *status, cudaStream_t s)
+{
+    const auto kern = vector_kernel<PT, ACC, V>;
+    const LaunchShape ls = cached_launch_shape(kern, VT, 0);
+    // Shares of a few chunks: enough for the prefetches to run ahead, small
+    // enough that the warps end together.
+    const long long warps = (long long)ls.sms * ls.occ * (VT / 32);
+    const long long chunks = ((long long)A.m + vector_chunk(V) - 1) / vector_chunk(V);
+    const long long share = vector_chunk(V) * std::min<long long>(8, std::max<long long>(1, chunks / (2 * warps)));
+    const long long need = (A.m + share - 1) / share;
+    hook_start(s);
+    kern<<<(int)((need * 32 + VT - 1) / VT), VT, 0, s>>>(
+        A.m, A.n, A.rowptr, A.col, static_cast<const typename PT::V *>(A.val), x, y, alpha, beta,
+        status, (int)share);
+    hook_stop(s);
 }
 
 template <typename PT, typename ACC>
@@ -41,25 +59,14 @@ void launch_vector_t(const CsrView &A, int V, double alpha, const typename PT::V
                      double beta, double *y, unsigned *status, cudaStream_t s)
 {
     if (A.m <= 0) return;
-    const auto *val = static_cast<const typename PT::V *>(A.val);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int CR = vector_chunk_rows(V, V < 4 ? V : 4);  // VectorShape<V>::CR
-    long long need = (((long long)A.m + CR - 1) / CR * 32 + VT - 1) / VT;  // a warp per chunk
-    int grid = (int)(need < (long long)sms * 64 ? need : (long long)sms * 64);
-#define SBB_VL(W)                                                                     \
-    case W:                                                                           \
-        vector_kernel<PT, ACC, W><<<grid, VT, 0, s>>>(A.m, A.n, A.rowptr, A.col, val, \
-                                                      x, y, alpha, beta, status);     \
-        break;
-    hook_start(s);
     switch (V) {
-        SBB_VL(2) SBB_VL(4) SBB_VL(8) SBB_VL(16) SBB_VL(32)
+    case 2: launch_vector_v<PT, ACC, 2>(A, alpha, x, beta, y, status, s); break;
+    case 4: launch_vector_v<PT, ACC, 4>(A, alpha, x, beta, y, status, s); break;
+    case 8: launch_vector_v<PT, ACC, 8>(A, alpha, x, beta, y, status, s); break;
+    case 16: launch_vector_v<PT, ACC, 16>(A, alpha, x, beta, y, status, s); break;
+    case 32: launch_vector_v<PT, ACC, 32>(A, alpha, x, beta, y, status, s); break;
     default: break;
     }
-    hook_stop(s);
-#undef SBB_VL
 }
 
 }  // namespace

@@ -11,91 +11,140 @@ namespace sbb {
 
 constexpr int kLongRow = 32;  // K2: rows longer than this in a segment are summed by the warp
 
-// K1 chunk shape: 32/V rows per sub-step, U sub-steps in flight together, at
-// most 32 rows (CR) per chunk.
-template <int V, int U_ = (V < 4 ? V : 4)> struct VectorShape {
-    static constexpr int RPW = 32 / V;
-    static constexpr int U = U_;
-    static constexpr int CR = RPW * U < 32 ? RPW * U : 32;
-};
-
-// K1: one chunk of CR consecutive rows [r0, r0 + CR) by one warp, V lanes per
-// row.  Lane l first loads rowptr[r0+l], rowptr[r0+l+1] and y[r0+l]
-// (coalesced, all in flight together).  Row q of the chunk is then reduced by
-// lane group q % (32/V) in sub-step q / (32/V); the U sub-steps run together,
-// their loads issued before any of them is summed, so a warp keeps U row
-// fetches per group in flight instead of one (U = UU changes only which loads
-// are in flight together, never a sum, so a caller picks it for its register
-// budget).  Per row the order of the sum is fixed for a given V: lane i of
-// the group adds the products of nnz lo+i, lo+i+V, lo+i+2V, ... in that order,
-// then the group's partial sums meet in an xor butterfly.  Lane l ends with
-// row r0+l's sum and writes y[r0+l] (one coalesced store per chunk).  All 32
-// lanes call this together (the shuffles use the full mask).
-template <typename PT, typename ACC, int V, int UU = (V < 4 ? V : 4)>
-__device__ __forceinline__ void vector_chunk(int r0, int m, int n, const int *__restrict__ rowptr,
-                                             const int *__restrict__ col,
-                                             const typename PT::V *__restrict__ val,
-                                             const typename PT::V *__restrict__ x,
-                                             double *__restrict__ y, double alpha, double beta,
-                                             uint64_t stream, unsigned &bad)
+// The sums of U rows held by a group of V lanes (acc[u] = this lane's part of
+// row u): lane li ends with the total of row li / (V / U).  At each step a
+// lane keeps half of the rows it still holds and hands the other half to the
+// lane o away, so U rows take U - 1 + log2(V / U) exchanges instead of
+// U * log2(V); a row's total is formed by the additions of the xor butterfly
+// over V lanes, so it has the butterfly's bits.
+template <int V, int U> __device__ __forceinline__ double group_row_sums(double (&acc)[U], int li)
 {
-    using S = VectorShape<V, UU>;
-    constexpr int RPW = S::RPW, U = S::U, CR = S::CR;
+#pragma unroll
+    for (int h = U / 2, o = V / 2; h > 0; h >>= 1, o >>= 1) {
+        const bool upper = li & o;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            const double send = upper ? acc[j] : acc[j + h];
+            const double keep = upper ? acc[j + h] : acc[j];
+            acc[j] = keep + __shfl_xor_sync(0xffffffffu, send, o, V);
+        }
+    }
+    double sum = acc[0];
+#pragma unroll
+    for (int o = V / U / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, V);
+    return sum;
+}
+
+// K1: rows [r0, r0 + count) by one warp, V lanes per row, a chunk of
+// vector_chunk(V) rows at a time.  Lane l loads rowptr[r+l], rowptr[r+l+1] and
+// y[r+l] of a chunk (coalesced) and ends with row r+l's sum, so y is written
+// with one coalesced store; row q of a chunk is reduced by lane group
+// q % (32/V), with the U rows of a group in flight together.  Three things run
+// ahead: the row pointers by one chunk; the nnz of the next chunk, when it has
+// at most kVectorPrefetch of them, into L2; and in a row the next V columns and
+// values, loaded while x is gathered for the current ones.  Per row the order
+// of the sum is fixed for a given V: lane i of the group adds the products of
+// nnz lo+i, lo+i+V, lo+i+2V, ... in that order, then the group's partial sums
+// meet in an xor butterfly.  All 32 lanes call this together (full-mask
+// shuffles).
+//
+// What bounds it: the latency of column and x loads in turn, and issue in the
+// row ends.  Against loads that wait for the rows before them, branches around
+// each load and a butterfly per row (us, FP64, beta = 0.5): 200k rows of 24 in
+// a band with 8, 16, 32 lanes 18.6, 18.8, 25.5 (21.2, 21.4, 26.9 before); 100k
+// rows of 100 in blocks with 16, 32 lanes 30.9, 30.9 (36.1, 31.4); 100k
+// power-law rows of 30 with 16, 32 lanes 64, 44 (81, 54).  Without the bound on
+// the L2 prefetch rows of 100 took 42, without the loads ahead in a row 38.
+constexpr unsigned kVectorPrefetch = 256;
+template <typename PT, typename ACC, int V>
+__device__ __forceinline__ void vector_rows(int r0, int count, int n,
+                                            const int *__restrict__ rowptr,
+                                            const int *__restrict__ col,
+                                            const typename PT::V *__restrict__ val,
+                                            const typename PT::V *__restrict__ x,
+                                            double *__restrict__ y, double alpha, double beta,
+                                            uint64_t stream, unsigned &bad)
+{
+    using T = typename PT::V;
+    constexpr int RPW = 32 / V, U = vector_rows_in_flight(V), CR = RPW * U;
     const int lane = threadIdx.x & 31, g = lane / V, li = lane & (V - 1);
-    const bool in = lane < CR && lane < m - r0;  // r0 < m: no overflow near INT_MAX
-    int rlo = 0, rhi = 0;
-    double yv = 0.0;
-    if (in) {
-        rlo = __ldg(rowptr + r0 + lane);
-        rhi = __ldg(rowptr + r0 + lane + 1);
-        if (beta != 0.0) yv = ld_y(y + r0 + lane, stream);
-    }
-    double out = 0.0;
-    // nnz indices are unsigned: with nnz up to 2^31 - 1 a lane's index runs
-    // to at most nnz - 1 + V (< 2^32), past the int range but never wrapping
+    int lo = 0, hi = 0, nlo = 0, nhi = 0;
+    // offsets from r0 stay in int
+    auto load_rows = [&](int at, int &a, int &b) {
+        a = b = 0;
+        if (lane < min(CR, count - at)) {
+            a = __ldg(rowptr + r0 + at + lane);
+            b = __ldg(rowptr + r0 + at + lane + 1);
+        }
+    };
+    auto prefetch = [&](int a, int b) {
+        const unsigned first = (unsigned)__shfl_sync(0xffffffffu, a, 0);
+        const unsigned end = __reduce_max_sync(0xffffffffu, (unsigned)b);
+        if (lane == 0 && end - first - 1u < kVectorPrefetch) {
+            prefetch_l2(col + first, 4 * (size_t)(end - first));
+            prefetch_l2(val + first, sizeof(T) * (size_t)(end - first));
+        }
+    };
+    load_rows(0, lo, hi);
+    if (CR < count) load_rows(CR, nlo, nhi);
+    prefetch(lo, hi);
 #pragma unroll 1
-    for (int j0 = 0; j0 * RPW < CR; j0 += U) {
-        unsigned k[U], hi[U];
+    for (int at = 0; at < count; at += CR) {
+        double yv = 0.0;
+        const bool in = lane < min(CR, count - at);
+        if (in && beta != 0.0) yv = ld_y(y + r0 + at + lane, stream);
+        if (at + CR < count) prefetch(nlo, nhi);
+        // nnz indices are unsigned: with nnz up to 2^31 - 1 a lane's index runs
+        // to at most nnz - 1 + V (< 2^32), past the int range but never wrapping
+        unsigned k[U], end[U];
         ACC acc[U];
+        bool any = false;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int q = (j0 + u) * RPW + g;
-            k[u] = (unsigned)__shfl_sync(0xffffffffu, rlo, q) + (unsigned)li;
-            hi[u] = (unsigned)__shfl_sync(0xffffffffu, rhi, q);
+            const int q = u * RPW + g;
+            k[u] = (unsigned)__shfl_sync(0xffffffffu, lo, q) + (unsigned)li;
+            end[u] = (unsigned)__shfl_sync(0xffffffffu, hi, q);
             acc[u].zero();
+            any |= k[u] < end[u];
         }
-        for (;;) {
-            bool any = false;
-            int c[U];
-            typename PT::V v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (k[u] < hi[u]) {
-                    c[u] = ld_stream(col + k[u]);
-                    v[u] = ld_stream(val + k[u]);
-                    any = true;
-                }
-            }
-            if (!any) break;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (k[u] < hi[u]) {
-                    acc[u].mac(v[u], gather_x(x, c[u], n, bad));
-                    k[u] += V;
-                }
-            }
-        }
+        lo = nlo;
+        hi = nhi;
+        if (at + 2 * CR < count) load_rows(at + 2 * CR, nlo, nhi);
+        int c[U];
+        T v[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            double sum = acc[u].get();
-#pragma unroll
-            for (int o = V / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, V);
-            // row q = (j0+u)*RPW + g lands in lane q
-            const double r = __shfl_sync(0xffffffffu, sum, (lane % RPW) * V);
-            if (lane / RPW == j0 + u) out = r;
+            c[u] = ld_stream_if(col + k[u], k[u] < end[u]);
+            v[u] = ld_stream_if(val + k[u], k[u] < end[u]);
         }
+        while (any) {
+            T xv[U], vn[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) xv[u] = gather_x_if(x, c[u], n, k[u] < end[u], bad);
+            any = false;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const unsigned kn = k[u] + V;
+                any |= kn < end[u];
+                c[u] = ld_stream_if(col + kn, kn < end[u]);
+                vn[u] = ld_stream_if(val + kn, kn < end[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (k[u] < end[u]) acc[u].mac(v[u], xv[u]);
+                v[u] = vn[u];
+                k[u] += V;
+            }
+        }
+        double part[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) part[u] = acc[u].get();
+        const double sum = group_row_sums<V, U>(part, li);
+        // row q = u*RPW + g lands in lane q
+        const double out =
+            __shfl_sync(0xffffffffu, sum, (lane % RPW) * V + (lane / RPW & (U - 1)) * (V / U));
+        if (in) st_y(y + r0 + at + lane, y_update(alpha, out, beta, yv), stream);
     }
-    if (in) st_y(y + r0 + lane, y_update(alpha, out, beta, yv), stream);
 }
 
 // Carry fix-up arithmetic shared by the standalone fix-up (k_fixup.cu) and

@@ -175,12 +175,12 @@ constexpr int kBatchMergeClass = 4; // classes 0..3: vector CSR with V = 4 << cl
 constexpr int kBatchTiledClass = 5; // CSR5-style tiles, sigma = kBatchSigma
 constexpr int kBatchSigma = 4;
 constexpr int kBatchTileGroup = 2;  // tiled class: tiles per work unit (one bulk copy)
-constexpr int kBatchClaim = 16;     // work units a warp claims per queue access
-constexpr int kBatchVectorNnz = 1024; // vector classes: about this many nnz per work unit
-constexpr int kBatchVectorU = 4;    // vector classes: rows of a lane group in flight together
-// Rows per K1 chunk for V lanes per row and U rows in flight per lane group
-// (VectorShape<V, U>::CR in spmv_device.cuh).
-constexpr int vector_chunk_rows(int V, int U) { return (32 / V) * U < 32 ? (32 / V) * U : 32; }
+constexpr int kBatchClaim = 16;     // most work units a warp claims per queue access
+constexpr int kBatchVectorNnz = 256; // vector classes: about this many nnz per work unit
+// Rows of a lane group of the vector kernel in flight together, and rows of
+// the warp: a chunk.
+constexpr int vector_rows_in_flight(int V) { return V < 4 ? V : 4; }
+constexpr int vector_chunk(int V) { return 32 / V * vector_rows_in_flight(V); }
 struct BatchMat {                   // one matrix of a batch, as the kernel sees it
     const int *rowptr, *col;
     const void *val;
@@ -222,22 +222,19 @@ bool tiled_view(const Plan *p, TiledView *v);
 // The plain-plan configuration of batch class cls (0 .. SBB_NUM_CLASSES-1).
 sbb_config batch_class_config(int cls);
 // Kernel families of the batch: one persistent kernel each, compiled with
-// only its family's code (so with that code's register budget): vector CSR
-// with 4 or 8 lanes, with 16 or 32 lanes, the merge class, the tiled class.
-enum { kFamVectorNarrow = 0, kFamVectorWide = 1, kFamMerge = 2, kFamTiled = 3,
-       kBatchFamilies = 4 };
+// only its family's code (so with that code's register budget): the vector
+// classes, the merge class, the tiled class.
+enum { kFamVector = 0, kFamMerge = 1, kFamTiled = 2, kBatchFamilies = 3 };
 inline int batch_family(int cls)
 {
-    return cls < 2 ? kFamVectorNarrow
-                   : (cls < kBatchMergeClass ? kFamVectorWide
-                                             : (cls == kBatchMergeClass ? kFamMerge : kFamTiled));
+    return cls < kBatchMergeClass ? kFamVector : (cls == kBatchMergeClass ? kFamMerge : kFamTiled);
 }
 int batch_max_ctas_per_sm(int fam);
 // Units [0, total) of the family's matrices mats[0..nmat) (unit0: nmat+1
-// prefix offsets), claimed from *queue.
+// prefix offsets), claimed `claim` at a time from *queue.
 void launch_batch(int fam, const BatchMat *mats, int nmat, const long long *unit0,
-                  long long total, unsigned long long *queue, unsigned *status, int grid,
-                  cudaStream_t s);
+                  long long total, int claim, unsigned long long *queue, unsigned *status,
+                  int grid, cudaStream_t s);
 void launch_batch_fixup(const BatchMat *mats, const BatchFix &F, long long total_slots,
                         cudaStream_t s);
 
