@@ -217,7 +217,7 @@ int sbb_batch_create(sbb_batch_t *out, const sbb_batch_item *items, int count, v
             M.crow = p->tile_row + 1;  // segment t carries into the row it ends in
             M.carry_val = p->carry_val;
             M.tiles = p->tiles;
-            units = p->tiles;
+            units = (p->tiles + kMergeGroup - 1) / kMergeGroup;
             if (!add_carries(i, p->tiles, p->runs)) {
                 batch_free(b);
                 return SBB_ERR_CUDA;

@@ -42,8 +42,7 @@ template <int FAM> struct FamShape {  // vector classes
     static constexpr int MINB = 4;
 };
 template <> struct FamShape<kFamMerge> {
-    static constexpr size_t kWarpBytes =
-        (sizeof(double) * SEG + sizeof(int) * (SEG + 1) + 127) / 128 * 128;
+    static constexpr size_t kWarpBytes = sizeof(double) * SEG;
     static constexpr int MINB = 4;
 };
 template <> struct FamShape<kFamTiled> {
@@ -151,12 +150,12 @@ batch_kernel(const BatchMat *__restrict__ mats, int nmat, const long long *__res
                 default: vector_unit<32>(M, local, bad); break;
                 }
             } else if constexpr (FAM == kFamMerge) {
-                unsigned char *wsm = warp_smem<FAM>();
-                merge_segment<ProdF64, AccF64, kBatchIpt>(
-                    local, M.n, M.rowptr, M.col, static_cast<const double *>(M.val), M.x, M.y,
-                    M.alpha, M.beta, M.tile_row, M.tile_nnz, M.carry_val, status,
-                    reinterpret_cast<double *>(wsm),
-                    reinterpret_cast<int *>(wsm + sizeof(double) * SEG), l2_evict_last(),
+                const int w0 = local * kMergeGroup;
+                merge_segments<ProdF64, AccF64, kBatchIpt>(
+                    w0, min(kMergeGroup, M.tiles - w0), M.n, M.rowptr, M.col,
+                    static_cast<const double *>(M.val), M.x, M.y, M.alpha, M.beta, M.tile_row,
+                    M.tile_nnz, M.carry_val, status,
+                    reinterpret_cast<double *>(warp_smem<FAM>()), l2_evict_last(),
                     l2_evict_first());
             } else {
                 int cur = 0;

@@ -10,8 +10,8 @@
 // restatement.
 //
 // Per warp segment (rows r0..r1-1 complete, row r1 open, nnz k0..k1-1):
-//   1. the row ends and the products val*x of the segment's nnz go to the
-//      warp's shared memory: coalesced streaming loads of col/val, every
+//   1. the products val*x of the segment's nnz go to the warp's shared memory
+//      and the row ends to its lanes: coalesced streaming loads of col/val, every
 //      load of the lane issued before any is used, x gathered through the
 //      read-only path with an L2 evict-last hint;
 //   2. each lane sums one row at a time straight from shared memory
@@ -21,6 +21,13 @@
 //   3. the part of row r1 inside the segment is the segment's carry, summed
 //      by the whole warp and added afterwards in a fixed order (k_fixup.cu).
 // The reduction order depends only on the matrix and IPT, never on timing.
+//
+// What bounds it: the L1 data pipe (gathers, products and row sums through
+// shared memory) and issue, 361 instructions a 192-item segment; on large
+// matrices HBM's latency came first.  Predicated loads without branches, row ends
+// in registers and, on large matrices, several segments a warp with their nnz
+// brought into L2 together: 60M nnz 385 -> 282 us, 7.6M nnz 47.5 -> 43.1 (FP32
+// storage 44.2 -> 38.5), 1.1M nnz 12.3 -> 11.5.
 #include <climits>
 
 #include "../sbb_internal.h"
@@ -90,27 +97,27 @@ merge_kernel(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
     using P = typename PT::P;
     constexpr int SEG = 32 * IPT;
     __shared__ P s_p[WPB][SEG];
-    __shared__ int s_re[WPB][SEG + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t keep = l2_evict_last(), streaming = l2_evict_first();
+    // segments [first, end), kMergeGroup at a time
+    auto run = [&](long long first, long long end) {
+        for (long long w = first; w < end; w += kMergeGroup)
+            merge_segments<PT, ACC, IPT>((int)w, (int)min((long long)kMergeGroup, end - w), n,
+                                         rowptr, col, val, x, y, alpha, beta, tile_row, tile_nnz,
+                                         carry_val, status, s_p[warp], keep, streaming);
+    };
     if (queue) {
         for (;;) {
             unsigned first = 0;
             if (lane == 0) first = atomicAdd(queue, (unsigned)item);
             first = __shfl_sync(0xffffffffu, first, 0);
             if (first >= (unsigned)tiles) break;
-            const int end = (int)min((unsigned long long)first + item, (unsigned long long)tiles);
-            for (int w = (int)first; w < end; ++w)
-                merge_segment<PT, ACC, IPT>(w, n, rowptr, col, val, x, y, alpha, beta, tile_row,
-                                            tile_nnz, carry_val, status, s_p[warp], s_re[warp],
-                                            keep, streaming);
+            run(first, min((long long)first + item, (long long)tiles));
         }
         return;
     }
-    for (int w = blockIdx.x * WPB + warp; w < tiles; w += gridDim.x * WPB)
-        merge_segment<PT, ACC, IPT>(w, n, rowptr, col, val, x, y, alpha, beta, tile_row,
-                                    tile_nnz, carry_val, status, s_p[warp], s_re[warp], keep,
-                                    streaming);
+    const long long first = ((long long)blockIdx.x * WPB + warp) * item;
+    run(first, min(first + item, (long long)tiles));
 }
 
 template <typename PT, typename ACC, int IPT>
@@ -120,14 +127,24 @@ void launch_merge_t(const CsrView &A, const MergeScratch &S, double alpha,
 {
     const auto *val = static_cast<const typename PT::V *>(A.val);
     if (S.tiles > 0) {
+        const auto kern = merge_kernel<PT, ACC, IPT>;
         long long blocks = (S.tiles + WPB - 1) / WPB;
         const bool queued = S.queue && S.persistent_ctas > 0 && S.persistent_ctas < blocks;
+        int item = S.queue_item > 0 ? S.queue_item : 1;
+        if (!queued) {
+            // kMergeGroup segments a warp when that still makes eight waves of
+            // blocks, else fewer, so that the last wave stays small (us for 4, 2
+            // and 1: 7.6M nnz 49.2, 45.0, 43.1; 60M nnz 282, -, 343)
+            const LaunchShape ls = cached_launch_shape(kern, NT, 0);
+            item = kMergeGroup;
+            while (item > 1 && blocks < 8LL * item * ls.sms * ls.occ) item >>= 1;
+            blocks = (S.tiles + (long long)item * WPB - 1) / ((long long)item * WPB);
+        }
         int grid = (int)(queued ? S.persistent_ctas : blocks);
         hook_start(s);
-        merge_kernel<PT, ACC, IPT><<<grid, NT, 0, s>>>(A.n, A.rowptr, A.col, val, x, y, alpha, beta,
-                                                       S.tile_row, S.tile_nnz, S.carry_val,
-                                                       S.tiles, status, queued ? S.queue : nullptr,
-                                                       S.queue_item > 0 ? S.queue_item : 1);
+        kern<<<grid, NT, 0, s>>>(A.n, A.rowptr, A.col, val, x, y, alpha, beta, S.tile_row,
+                                 S.tile_nnz, S.carry_val, S.tiles, status,
+                                 queued ? S.queue : nullptr, item);
         hook_stop(s);
         launch_fixup(A.m, S.tile_row + 1, S.carry_val, S.tiles, *S.runs, alpha, y,
                      queued ? S.queue : nullptr, s, S.runs_count);

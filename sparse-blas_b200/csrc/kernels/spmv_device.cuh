@@ -193,110 +193,109 @@ __device__ __forceinline__ double warp_range_sum(const P *s_p, int lo, int hi, i
     return warp_sum(acc.get());
 }
 
+// K2: `count` (at most kMergeGroup) consecutive merge-path segments by one
+// warp, the first of them segment w0.  Lane l reads the coordinates of segment
+// w0 + l, all at once, and the nnz of the whole group (contiguous) are brought
+// into L2 together, so the segments after the first find them there.
 template <typename PT, typename ACC, int IPT>
-__device__ __forceinline__ void merge_segment(
-    int w, int n, const int *__restrict__ rowptr, const int *__restrict__ col,
+__device__ __forceinline__ void merge_segments(
+    int w0, int count, int n, const int *__restrict__ rowptr, const int *__restrict__ col,
     const typename PT::V *__restrict__ val, const typename PT::V *__restrict__ x,
     double *__restrict__ y, double alpha, double beta, const int *__restrict__ tile_row,
     const int *__restrict__ tile_nnz, double *__restrict__ carry_val, unsigned *status,
-    typename PT::P *s_p, int *s_re, uint64_t keep, uint64_t streaming)
+    typename PT::P *s_p, uint64_t keep, uint64_t streaming)
 {
-    using P = typename PT::P;
     using V = typename PT::V;
     constexpr int SEG = 32 * IPT;
     const int lane = threadIdx.x & 31;
-    const int r0 = __ldg(tile_row + w), r1 = __ldg(tile_row + w + 1);
-    const int k0 = __ldg(tile_nnz + w), k1 = __ldg(tile_nnz + w + 1);
-    const int nrows = r1 - r0, nz = k1 - k0;
-    if (nrows < 0 || nz < 0 || nrows + nz > SEG) {  // corrupt coordinates
-        if (lane == 0) atomicOr(status, ST_BAD_TILE);
-        return;
+    int crow = 0, cnnz = 0;
+    if (lane <= count) {
+        crow = __ldg(tile_row + w0 + lane);
+        cnnz = __ldg(tile_nnz + w0 + lane);
     }
     unsigned bad = 0;
-    // y of the first 32 rows, early: the beta*y read then is off the tail
-    double ypre = 0.0;
-    if (beta != 0.0 && lane < nrows) ypre = ld_y(y + r0 + lane, streaming);
-
-    // 1. row ends and products (every load of the lane in flight together)
-    int cc[IPT];
-    V vv[IPT];
-#pragma unroll
-    for (int j = 0; j < IPT; ++j) {
-        const int i = lane + 32 * j;
-        if (i < nz) {
-            cc[j] = ld_stream(col + k0 + i);
-            vv[j] = ld_stream(val + k0 + i);
+    if (count > 1) {
+        const int a = __shfl_sync(0xffffffffu, cnnz, 0), b = __shfl_sync(0xffffffffu, cnnz, count);
+        if (lane == 0 && b > a && b - a <= SEG * kMergeGroup) {
+            prefetch_l2(col + a, 4 * (size_t)(b - a));
+            prefetch_l2(val + a, sizeof(V) * (size_t)(b - a));
         }
     }
+#pragma unroll 1
+    for (int g = 0; g < count; ++g) {
+        const int r0 = __shfl_sync(0xffffffffu, crow, g), r1 = __shfl_sync(0xffffffffu, crow, g + 1);
+        const int k0 = __shfl_sync(0xffffffffu, cnnz, g), k1 = __shfl_sync(0xffffffffu, cnnz, g + 1);
+        const int nrows = r1 - r0, nz = k1 - k0;
+        if (nrows < 0 || nz < 0 || nrows + nz > SEG) {  // corrupt coordinates
+            if (lane == 0) atomicOr(status, ST_BAD_TILE);
+            continue;
+        }
+        // 1. products to shared memory: every load of the lane in flight
+        // together, with the first 32 row ends and their y
+        int c[IPT];
+        V v[IPT];
 #pragma unroll
-    for (int j = 0; j < IPT; ++j) {
-        const int i = lane + 32 * j;
-        if (i < nrows) s_re[i] = __ldg(rowptr + r0 + 1 + i);
-    }
-    V xv[IPT];
+        for (int j = 0; j < IPT; ++j) {
+            const bool p = lane + 32 * j < nz;
+            c[j] = ld_stream_if(col + k0 + lane + 32 * j, p);
+            v[j] = ld_stream_if(val + k0 + lane + 32 * j, p);
+        }
+        int end = k0;  // end of row r0 + b + lane, for the 32 rows from b
+        if (lane < nrows) end = __ldg(rowptr + r0 + 1 + lane);
+        double yv = 0.0;
+        if (beta != 0.0 && lane < nrows) yv = ld_y(y + r0 + lane, streaming);
+        V xv[IPT];
 #pragma unroll
-    for (int j = 0; j < IPT; ++j) {
-        const int i = lane + 32 * j;
-        if (i < nz) {
-            if ((unsigned)cc[j] < (unsigned)n) {
-                xv[j] = ld_keep(x + cc[j], keep);
-            } else {
-                bad = 1u;
-                xv[j] = V(0);
+        for (int j = 0; j < IPT; ++j) {
+            const bool p = lane + 32 * j < nz, ok = (unsigned)c[j] < (unsigned)n;
+            bad |= p && !ok;
+            xv[j] = ld_keep_if(x + c[j], p && ok, keep);
+        }
+#pragma unroll
+        for (int j = 0; j < IPT; ++j)
+            if (lane + 32 * j < nz) s_p[lane + 32 * j] = PT::make(v[j], xv[j]);
+        __syncwarp();
+
+        // 2. complete rows r0 .. r1-1: lane per row, long rows by the warp
+        int before = 0;  // where row r0 + b starts (it may have started before k0)
+        for (int b = 0; b < nrows; b += 32) {
+            const int i = b + lane;
+            if (b > 0) {
+                if (i < nrows) end = __ldg(rowptr + r0 + 1 + i);
+                if (beta != 0.0 && i < nrows) yv = ld_y(y + r0 + i, streaming);
             }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < IPT; ++j) {
-        const int i = lane + 32 * j;
-        if (i < nz) s_p[i] = PT::make(vv[j], xv[j]);
-    }
-    if (bad) atomicOr(status, ST_BAD_COL);
-    __syncwarp();
-
-    // 2. complete rows r0 .. r1-1: lane per row, long rows by the warp
-    for (int b = 0; b < nrows; b += 32) {
-        const int i = b + lane;
-        int lo = 0, hi = 0;
-        if (i < nrows) {
-            lo = i == 0 ? 0 : s_re[i - 1] - k0;  // row r0 may have started before k0
-            hi = s_re[i] - k0;
             // a valid row pointer keeps 0 <= lo <= hi <= nz; clamping makes a
             // corrupt one harmless (wrong sums, no out-of-range reads)
-            lo = min(max(lo, 0), nz);
-            hi = min(max(hi, lo), nz);
-        }
-        const bool is_long = hi - lo > kLongRow;
-        if (i < nrows && !is_long) {
-            ACC acc;
-            acc.zero();
-            for (int k = lo; k < hi; ++k) acc.add(s_p[k]);
-            double *yp = y + r0 + i;
-            const double v = y_update(alpha, acc.get(), beta,
-                                      beta == 0.0 ? 0.0 : (b == 0 ? ypre : ld_y(yp, streaming)));
-            st_y(yp, v, streaming);
-        }
-        unsigned longs = __ballot_sync(0xffffffffu, i < nrows && is_long);
-        while (longs) {
-            const int src = __ffs(longs) - 1;
-            longs &= longs - 1;
-            const int llo = __shfl_sync(0xffffffffu, lo, src);
-            const int lhi = __shfl_sync(0xffffffffu, hi, src);
-            const double s = warp_range_sum<ACC>(s_p, llo, lhi, lane);
-            if (lane == src) {
-                double *yp = y + r0 + i;
-                const double v = y_update(alpha, s, beta,
-                                          beta == 0.0 ? 0.0 : (b == 0 ? ypre : ld_y(yp, streaming)));
-                st_y(yp, v, streaming);
+            int hi = min(max(end - k0, 0), nz), lo = __shfl_up_sync(0xffffffffu, hi, 1);
+            if (lane == 0) lo = before;
+            hi = max(hi, lo);
+            const bool in = i < nrows, is_long = hi - lo > kLongRow;
+            double sum = 0.0;
+            if (in && !is_long) {
+                ACC acc;
+                acc.zero();
+#pragma unroll 4
+                for (int k = lo; k < hi; ++k) acc.add(s_p[k]);
+                sum = acc.get();
             }
+            unsigned longs = __ballot_sync(0xffffffffu, in && is_long);
+            while (longs) {
+                const int src = __ffs(longs) - 1;
+                longs &= longs - 1;
+                const int llo = __shfl_sync(0xffffffffu, lo, src);
+                const int lhi = __shfl_sync(0xffffffffu, hi, src);
+                const double t = warp_range_sum<ACC>(s_p, llo, lhi, lane);
+                if (lane == src) sum = t;
+            }
+            if (in) st_y(y + r0 + i, y_update(alpha, sum, beta, yv), streaming);
+            before = __shfl_sync(0xffffffffu, hi, min(31, nrows - b - 1));
         }
+        // 3. carry: the part of row r1 inside this segment
+        const double t = warp_range_sum<ACC>(s_p, before, nz, lane);
+        if (lane == 0) carry_val[w0 + g] = t;
+        __syncwarp();  // shared memory is reused by the next segment
     }
-    // 3. carry: the part of row r1 inside this segment
-    const int clo = nrows > 0 ? min(max(s_re[nrows - 1] - k0, 0), nz) : 0;
-    const double c = warp_range_sum<ACC>(s_p, clo, nz, lane);
-    if (lane == 0) carry_val[w] = c;
-    __syncwarp();  // shared memory is reused by this warp's next segment
+    if (bad) atomicOr(status, ST_BAD_COL);
 }
-
 
 }  // namespace sbb

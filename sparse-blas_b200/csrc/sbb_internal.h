@@ -94,6 +94,7 @@ LaunchShape cached_launch_shape(K kern, int threads, size_t smem)
 
 // ---- kernel launchers (defined in the .cu files) ---------------------------
 constexpr int kMergeThreads = 256;
+constexpr int kMergeGroup = 4;      // most consecutive segments a warp takes together
 // Tile plans take at most this many rows: row counts and segment ranks plus
 // a tile's offsets stay in int.  The automatic and learned choices use the
 // merge path above it.
