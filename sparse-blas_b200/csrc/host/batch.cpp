@@ -167,11 +167,16 @@ int sbb_batch_create(sbb_batch_t *out, const sbb_batch_item *items, int count, v
         fix_mat.push_back(i);
         tile0.push_back(tile0.back() + slots);
         std::vector<int> f, l;
-        if (!fetch(f, R.run_first, R.n_runs) || !fetch(l, R.run_len, R.n_runs)) return false;
-        for (int r = 0; r < R.n_runs; r++) {
-            run_mat.push_back(i);
-            run_first.push_back(f[r]);
-            run_len.push_back(l[r]);
+        // long runs from the front of the lists, short ones from the back
+        const int cap = slots / 2 + 1;
+        for (int part = 0; part < 2; part++) {
+            const int at = part ? cap - R.n_short : 0, cnt = part ? R.n_short : R.n_long;
+            if (!fetch(f, R.run_first + at, cnt) || !fetch(l, R.run_len + at, cnt)) return false;
+            for (int r = 0; r < cnt; r++) {
+                run_mat.push_back(i);
+                run_first.push_back(f[r]);
+                run_len.push_back(l[r]);
+            }
         }
         return true;
     };

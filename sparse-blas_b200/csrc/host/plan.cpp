@@ -39,8 +39,6 @@ int plan_launches(const Plan *p)
     }
 }
 
-void launch_rowptr_check(const int *rp, int m, int nnz, unsigned *status, cudaStream_t s);
-
 // Lanes per row of the row slices: enough that a row takes about 8 to 32 steps
 // (us for 1, 2, 4, 8 lanes: rows of 6 11.8, 12.4, 15.7, -; of 24 15.5, 14.4,
 // 15.8, 19.0; of 50 -, 15.4, 15.0, 16.3; of 100 -, 27.1, 26.4, 26.6), and more
@@ -201,11 +199,10 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
     int rc;
     if ((rc = dalloc(&p->status, 4, s, &p->scratch_bytes))) return rc;
     SBB_CUDA(cudaMemsetAsync(p->status, 0, 4 * sizeof(unsigned), s));
-    int *stats = reinterpret_cast<int *>(p->status + 2);
-    bool want_stats = validate && (cfg == nullptr || cfg->kernel == SBB_KERNEL_AUTO);
+    const bool want_stats = validate && (cfg == nullptr || cfg->kernel == SBB_KERNEL_AUTO);
     if (validate) {
-        launch_rowptr_check(p->rowptr, p->m, p->nnz, p->status, s);
-        if (want_stats) launch_row_stats(p->rowptr, p->m, stats, s);
+        launch_csr_check(p->rowptr, p->m, p->nnz, nullptr, p->n, p->status,
+                         reinterpret_cast<int *>(p->status + 2), s);
         unsigned h[4];
         SBB_CUDA(cudaMemcpyAsync(h, p->status, sizeof(h), cudaMemcpyDeviceToHost, s));
         SBB_CUDA(cudaStreamSynchronize(s));
@@ -216,7 +213,6 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
         }
         p->max_row = (int)h[2];
         p->empty_rows = (int)h[3];
-        SBB_CUDA(cudaMemsetAsync(p->status, 0, 4 * sizeof(unsigned), s));
     }
     sbb_config c{};
     if (cfg) c = *cfg;
@@ -305,9 +301,8 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
         if (tiles > 0) {
             launch_merge_partition(p->rowptr, p->m, p->base, p->nnz, items, p->tiles, p->tile_row,
                                    p->tile_nnz, s);
-            rc = p->device_runs
-                     ? carry_runs_build_device(p->tile_row + 1, p->tiles, p->m, &p->runs, s)
-                     : carry_runs_build(p->tile_row + 1, p->tiles, p->m, &p->runs, s);
+            rc = carry_runs_build(p->tile_row + 1, p->tiles, p->m, &p->runs, s);
+            if (!rc && !p->device_runs) rc = carry_runs_counts(&p->runs, s);
             if (rc) return rc;
             p->scratch_bytes += p->runs.bytes;
         }
@@ -401,7 +396,7 @@ int plan_run(Plan *p, double alpha, const void *x, double beta, double *y, cudaS
                           p->status, s);
         break;
     case SBB_KERNEL_MERGE: {
-        MergeScratch S{p->tile_row, p->tile_nnz, p->carry_val, &p->runs, p->runs.count, p->tiles,
+        MergeScratch S{p->tile_row, p->tile_nnz, p->carry_val, &p->runs, p->tiles,
                        p->queue, p->persistent_ctas, merge_queue_item(*p)};
         if (p->f32)
             launch_merge_f32(A, p->ipt, S, alpha, static_cast<const float *>(x), beta, y,

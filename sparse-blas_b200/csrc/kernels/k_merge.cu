@@ -147,7 +147,7 @@ void launch_merge_t(const CsrView &A, const MergeScratch &S, double alpha,
                                  queued ? S.queue : nullptr, item);
         hook_stop(s);
         launch_fixup(A.m, S.tile_row + 1, S.carry_val, S.tiles, *S.runs, alpha, y,
-                     queued ? S.queue : nullptr, s, S.runs_count);
+                     queued ? S.queue : nullptr, s);
     }
 }
 

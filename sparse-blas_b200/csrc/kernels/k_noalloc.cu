@@ -40,7 +40,7 @@ constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 constexpr size_t kCoordBytes = align256(sizeof(int) * (kMaxSegments + 1));
 constexpr size_t kCarryBytes = align256(sizeof(double) * kMaxSegments);
 constexpr size_t kRunBytes = align256(sizeof(int) * (kMaxSegments / 2 + 1));
-constexpr size_t kWordBytes = 256;  // run count, status
+constexpr size_t kWordBytes = 256;  // run counts, status
 constexpr size_t kScratchBytes = 2 * kCoordBytes + kCarryBytes + 2 * kRunBytes + kWordBytes;
 
 // The scratch.  In host code this name is only a host-side stand-in: kernels
@@ -118,7 +118,7 @@ extern "C" int sbb_spmv_merge_noalloc(int m, int n, int nnz, const int *d_rowptr
     int *run_len = reinterpret_cast<int *>(base + 2 * kCoordBytes + kCarryBytes + kRunBytes);
     int *words = reinterpret_cast<int *>(base + 2 * kCoordBytes + kCarryBytes + 2 * kRunBytes);
     int *run_count = words;
-    unsigned *status = reinterpret_cast<unsigned *>(words + 1);
+    unsigned *status = reinterpret_cast<unsigned *>(words + 2);
     const int tiles = (int)((items + kItems - 1) / kItems);
 
     // The array keeps the previous call's contents: clear what must start at 0.
@@ -129,7 +129,8 @@ extern "C" int sbb_spmv_merge_noalloc(int m, int n, int nnz, const int *d_rowptr
     CarryRuns runs;
     runs.run_first = run_first;
     runs.run_len = run_len;
-    MergeScratch S{tile_row, tile_nnz, carry_val, &runs, run_count, tiles, nullptr, 0, 1};
+    runs.count = run_count;
+    MergeScratch S{tile_row, tile_nnz, carry_val, &runs, tiles, nullptr, 0, 1};
     launch_merge(A, kIpt, S, alpha, d_x, beta, d_y, status, s);
     SBB_CUDA(cudaGetLastError());
     return SBB_OK;

@@ -502,6 +502,7 @@ int rows_build(Plan *p, cudaStream_t s)
             p->rowptr, m, kRowsShapes[R->shape].nmax, nullptr, offset, R->desc, R->carry_row);
     if (nblk > 0) {
         int rc = carry_runs_build(R->carry_row, nblk, m, &R->runs, s);
+        if (!rc) rc = carry_runs_counts(&R->runs, s);
         if (rc) return rc;
         p->scratch_bytes += R->runs.bytes;
     }

@@ -131,8 +131,8 @@ void launch_blob_fill(int sigma, const int *rp, const int *col, const void *val,
     }
 }
 
-// Row-start bits (one per nnz, original order within the tile) and
-// non-empty flags.
+// Row-start bits (one per nnz, original order within the tile) and, unless
+// null, non-empty flags.
 __global__ void starts_kernel(const int *__restrict__ rp, int m, int sigma, int vbytes,
                               unsigned char *__restrict__ blob, int *__restrict__ nonempty)
 {
@@ -142,7 +142,7 @@ __global__ void starts_kernel(const int *__restrict__ rp, int m, int sigma, int 
          r += (long long)gridDim.x * blockDim.x) {
         int lo = rp[r], hi = rp[r + 1];
         int ne = hi > lo;
-        nonempty[r] = ne;
+        if (nonempty) nonempty[r] = ne;
         if (ne) {
             long long k = lo - rp[0];
             long long t = k / TILE, q = k % TILE;
@@ -504,11 +504,15 @@ int tiled_build(Plan *p, cudaStream_t s)
     };
     const int m = p->m;
     int *flag = nullptr, *rank = nullptr;
+    // Without empty rows (known of a validated plan) a row's rank among the
+    // non-empty ones is its index, and nothing has to be counted.
+    const bool ranked = p->empty_rows != 0;
     bool ok = al((void **)&T->blob, T->tile_bytes * (size_t)tiles) &&
               al((void **)&T->tile_seg, sizeof(int) * (tiles + 1)) &&
               al((void **)&T->carry_row, sizeof(int) * tiles) &&
               al((void **)&T->carry_val, sizeof(double) * tiles) &&
-              al((void **)&flag, sizeof(int) * (m + 1)) && al((void **)&rank, sizeof(int) * (m + 1));
+              (!ranked || (al((void **)&flag, sizeof(int) * (m + 1)) &&
+                           al((void **)&rank, sizeof(int) * (m + 1))));
     if (!ok) {
         set_error("tiled plan: device allocation failed");
         return SBB_ERR_NOMEM;
@@ -523,16 +527,22 @@ int tiled_build(Plan *p, cudaStream_t s)
     }
     if (m > 0)
         starts_kernel<<<grid_for(m, 256), 256, 0, s>>>(p->rowptr, m, T->sigma, vbytes, T->blob, flag);
-    // rank[r] = number of non-empty rows before r (rank[m] = count)
-    SBB_CUDA(cudaMemsetAsync(flag + m, 0, sizeof(int), s));
-    size_t tmp_bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flag, rank, m + 1, s);
+    int count = m;
     void *tmp = nullptr;
-    if (!al(&tmp, tmp_bytes)) return SBB_ERR_NOMEM;
-    cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flag, rank, m + 1, s);
-    int count = 0;
-    SBB_CUDA(cudaMemcpyAsync(&count, rank + m, sizeof(int), cudaMemcpyDeviceToHost, s));
-    SBB_CUDA(cudaStreamSynchronize(s));
+    if (ranked) {
+        // rank[r] = number of non-empty rows before r (rank[m] = count)
+        SBB_CUDA(cudaMemsetAsync(flag + m, 0, sizeof(int), s));
+        size_t tmp_bytes = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flag, rank, m + 1, s);
+        if (!al(&tmp, tmp_bytes)) return SBB_ERR_NOMEM;
+        cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flag, rank, m + 1, s);
+        if (p->empty_rows > 0) {
+            count = m - p->empty_rows;
+        } else {
+            SBB_CUDA(cudaMemcpyAsync(&count, rank + m, sizeof(int), cudaMemcpyDeviceToHost, s));
+            SBB_CUDA(cudaStreamSynchronize(s));
+        }
+    }
     T->n_empty = m - count;
     if (T->n_empty > 0) {
         if (!al((void **)&T->ne, sizeof(int) * (count + 1)) ||
@@ -549,12 +559,12 @@ int tiled_build(Plan *p, cudaStream_t s)
         tile_header_kernel<<<(int)(((long long)T->tiles * 32 + 255) / 256), 256, 0, s>>>(
             T->tile_seg, T->sigma, vbytes, T->tiles, T->blob);
         int rc = carry_runs_build(T->carry_row, T->tiles, m, &T->runs, s);
+        if (!rc && !p->device_runs) rc = carry_runs_counts(&T->runs, s);
         if (rc) return rc;
         p->scratch_bytes += T->runs.bytes;
     }
-    SBB_CUDA(cudaFreeAsync(tmp, s));
-    SBB_CUDA(cudaFreeAsync(flag, s));
-    SBB_CUDA(cudaFreeAsync(rank, s));
+    for (void *q : {tmp, (void *)flag, (void *)rank})
+        if (q) SBB_CUDA(cudaFreeAsync(q, s));
     SBB_CUDA(cudaGetLastError());
     return SBB_OK;
 }

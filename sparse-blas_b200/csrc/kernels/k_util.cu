@@ -1,6 +1,8 @@
 // k_util.cu — small device kernels around the SpMV: row-pointer narrowing
 // and validation, row-length statistics, and the boundary-piece sums used by
 // the drop-in entry points.
+#include <algorithm>
+
 #include "../sbb_internal.h"
 #include "common.cuh"
 
@@ -29,38 +31,36 @@ __global__ void rowptr_narrow_kernel(const long long *__restrict__ src, int *__r
     if (bad) atomicOr(status, ST_BAD_ROWPTR);
 }
 
-__global__ void rowptr_check_kernel(const int *__restrict__ rp, int m, int nnz,
-                                    unsigned *status)
+__global__ void __launch_bounds__(256)
+csr_check_kernel(const int *__restrict__ rp, int m, int nnz, const int *__restrict__ col, int n,
+                 unsigned *status, int *stats)
 {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long stride = (long long)gridDim.x * blockDim.x;
-    bool bad = false;
-    for (; i <= m; i += stride) {
-        int v = rp[i];
-        if (v < 0 || v > nnz) bad = true;
-        if (i < m && v > rp[i + 1]) bad = true;
-        if (i == 0 && v != 0) bad = true;
-        if (i == m && v != nnz) bad = true;
-    }
-    if (bad) atomicOr(status, ST_BAD_ROWPTR);
-}
-
-__global__ void row_stats_kernel(const int *__restrict__ rp, int m, int *out)
-{
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    unsigned bad = 0;
     int mx = 0, empty = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-         i += (long long)gridDim.x * blockDim.x) {
-        int len = rp[i + 1] - rp[i];
-        mx = max(mx, len);
-        empty += (len == 0);
+    for (long long i = first; i <= m; i += stride) {
+        const int v = __ldg(rp + i);
+        if (v < 0 || v > nnz) bad |= ST_BAD_ROWPTR;
+        if (i == 0 && v != 0) bad |= ST_BAD_ROWPTR;
+        if (i == m && v != nnz) bad |= ST_BAD_ROWPTR;
+        if (i < m) {
+            const int w = __ldg(rp + i + 1);
+            if (v > w) bad |= ST_BAD_ROWPTR;
+            mx = max(mx, w - v);
+            empty += w == v;
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        empty += __shfl_xor_sync(0xffffffffu, empty, o);
-    }
+    if (col)
+        for (long long k = first; k < nnz; k += stride)
+            if ((unsigned)__ldg(col + k) >= (unsigned)n) bad |= ST_BAD_COL;
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    empty = __reduce_add_sync(0xffffffffu, empty);
+    bad = __reduce_or_sync(0xffffffffu, bad);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(out, mx);
-        if (empty) atomicAdd(out + 1, empty);
+        if (mx > 0) atomicMax(stats, mx);
+        if (empty) atomicAdd(stats + 1, empty);
+        if (bad) atomicOr(status, bad);
     }
 }
 
@@ -103,15 +103,12 @@ void launch_rowptr_narrow(const long long *src, int *dst, int m, long long nnz,
     rowptr_narrow_kernel<<<grid_for((long long)m + 1, 256), 256, 0, s>>>(src, dst, m, nnz, status);
 }
 
-void launch_rowptr_check(const int *rp, int m, int nnz, unsigned *status, cudaStream_t s)
+void launch_csr_check(const int *rp, int m, int nnz, const int *col, int n, unsigned *status,
+                      int *stats, cudaStream_t s)
 {
-    rowptr_check_kernel<<<grid_for((long long)m + 1, 256), 256, 0, s>>>(rp, m, nnz, status);
-}
-
-void launch_row_stats(const int *rowptr, int m, int *out, cudaStream_t s)
-{
-    if (m <= 0) return;
-    row_stats_kernel<<<grid_for(m, 256), 256, 0, s>>>(rowptr, m, out);
+    const long long work = std::max<long long>((long long)m + 1, col ? nnz : 0);
+    csr_check_kernel<<<(int)std::min<long long>((work + 255) / 256, 148 * 16), 256, 0, s>>>(
+        rp, m, nnz, col, n, status, stats);
 }
 
 void launch_pieces(const long long *lo, const long long *hi, int npieces, const int *col,

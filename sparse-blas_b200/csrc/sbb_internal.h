@@ -110,9 +110,11 @@ struct CsrView {          // rows [0, m) of a CSR matrix; offsets are absolute
 // rowptr int64 -> int32 with validation (monotone, within [0, nnz]).
 void launch_rowptr_narrow(const long long *src, int *dst, int m, long long nnz,
                           unsigned *status, cudaStream_t s);
-void launch_rowptr_check(const int *rp, int m, int nnz, unsigned *status, cudaStream_t s);
-// Row-length statistics: out[0] = max row length, out[1] = #empty rows.
-void launch_row_stats(const int *rowptr, int m, int *out, cudaStream_t s);
+// The same checks on an int32 row pointer, with row-length statistics: stats[0] =
+// max row length, stats[1] = #empty rows (of a valid pointer; zeroed before).
+// With columns (col non-null) also that every one is in [0, n).
+void launch_csr_check(const int *rp, int m, int nnz, const int *col, int n, unsigned *status,
+                      int *stats, cudaStream_t s);
 
 // K1: vector CSR, V lanes per row.
 void launch_vector(const CsrView &A, int V, double alpha, const double *x,
@@ -126,26 +128,25 @@ void launch_vector_f32(const CsrView &A, int V, double alpha, const float *x,
 // Runs of at most this many carries are summed by one warp, longer ones by a
 // block (spmv_device.cuh: fixup_run_warp, fixup_partial).
 constexpr int kWarpRunMax = 1024;
-struct CarryRuns {
+struct CarryRuns {   // run_first / run_len: long runs from the front, short ones from the back
     int *run_first = nullptr, *run_len = nullptr;
-    int n_runs = 0;
-    int n_long = 0;   // runs longer than kWarpRunMax, listed first
-    int *count = nullptr;  // device-built lists: the run count, on the device only
+    int n_long = 0, n_short = 0;  // runs of more than kWarpRunMax carries, and the others
+    int *count = nullptr;  // non-null: the two counts are on the device only
     size_t bytes = 0;
 };
+// Lists the runs on the device, in the order the marking kernel finds them,
+// without any host synchronisation; the counts stay there (R->count).
 int carry_runs_build(const int *carry_row, int T, int m, CarryRuns *R, cudaStream_t s);
-// The same lists built without any host synchronisation: runs in the order
-// the marking kernel found them, their count left on the device (R->count).
-int carry_runs_build_device(const int *carry_row, int T, int m, CarryRuns *R, cudaStream_t s);
+// Brings the counts to the host (one synchronisation), so that the fix-up is
+// launched with as many blocks as there are runs.
+int carry_runs_counts(CarryRuns *R, cudaStream_t s);
 void carry_runs_free(CarryRuns *R, cudaStream_t s);
-// Marks the runs on the device only; the count stays in *dev_count.
+// The marking alone: T / 2 + 1 entries in each list, two counts (zeroed).
 void launch_runs_mark(const int *carry_row, int T, int m, int *run_first, int *run_len,
                       int *dev_count, cudaStream_t s);
 // Adds the carries to y in a fixed order; also rearms `queue` when non-null.
-// dev_count non-null: the run count is read on the device (R.n_runs unused).
 void launch_fixup(int m, const int *carry_row, const double *carry_val, int T,
-                  const CarryRuns &R, double alpha, double *y, unsigned *queue, cudaStream_t s,
-                  const int *dev_count = nullptr);
+                  const CarryRuns &R, double alpha, double *y, unsigned *queue, cudaStream_t s);
 
 // K2: merge path.  One warp per segment of 32*IPT merge items.
 int merge_ipt_supported(int ipt);
@@ -156,7 +157,6 @@ struct MergeScratch {
     const int *tile_row, *tile_nnz;   // tiles+1 coordinates; tile t carries row tile_row[t+1]
     double *carry_val;                // tiles
     const CarryRuns *runs;
-    const int *runs_count;            // non-null: run count kept on the device
     int tiles;
     unsigned *queue;                  // persistent form: [0] = next segment to claim
     int persistent_ctas;              // 0 = one CTA per tile
@@ -276,10 +276,10 @@ struct Plan {
     int vector_width = 0;    // K1
     int ipt = 0;             // K2
     int persistent = 0;      // K2 persistent CTAs per SM (0 = off)
-    bool device_runs = false; // K2: carry runs built and counted on the device (no host sync)
+    bool device_runs = false; // K2, K3: carry runs counted on the device (no host sync)
     long long queue_nnz = 0; // K2 persistent form: nnz per queue item (0 = one segment)
     int tile_sigma = 0;      // K3
-    int max_row = 0, empty_rows = 0;
+    int max_row = 0, empty_rows = -1;  // of a validated plan (else 0, -1)
     // device scratch owned by the plan
     int *tile_row = nullptr, *tile_nnz = nullptr;
     double *carry_val = nullptr;
