@@ -60,7 +60,9 @@ int spMV_mgpu_v2(int m, int n, long long nnz, double *alpha, double *csrVal,
  * SparseBLAS/src/csr5_kernel.cu:12-32).  DEVICE pointers, int32 row pointer.
  * Unlike the reference, alpha and beta are honoured
  * (the reference drops them: include/detail/cuda/csr5_spmv_cuda.h:22,
- * include/anonymouslib_cuda.h:281) and the caller's col/val are not modified. */
+ * include/anonymouslib_cuda.h:281) and the caller's col/val are not modified.
+ * A call checks the matrix and multiplies once, on the caller's arrays; the
+ * tile format, which pays when it is kept, is SBB_KERNEL_TILED below. */
 int csr5_kernel(int m, int n, int nnz, double *alpha, double *csrVal,
                 int *csrRowPtr, int *csrColIndex, double *x, double *beta,
                 double *y);

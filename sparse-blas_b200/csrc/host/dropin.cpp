@@ -658,19 +658,66 @@ double min_free_gb(int ngpu)
     return best;
 }
 
+// One product with a matrix that is seen once: no tiles are built, because
+// writing and reading a copy of the matrix costs more than the product gains
+// (us a call with tiles and without: 15M nnz of a circuit 351 and 167, 1.1M nnz
+// 193 and 82, 4.8M nnz of even rows 207 and 75, 12M nnz in 4,284 rows 301 and
+// 123).  One pass checks the row pointer and the columns and takes the
+// row statistics; then even rows go to the vector kernel and others to the merge
+// path, both on the caller's arrays.
 int csr5_entry(int m, int n, int nnz, double *alpha, double *csrVal, int *csrRowPtr,
                int *csrColIndex, double *x, double *beta, double *y)
 {
-    if (!alpha || !beta) return -1;
-    sbb_config cfg{};
-    cfg.kernel = SBB_KERNEL_TILED;
-    sbb_plan_t plan = nullptr;
-    if (sbb_plan_create(&plan, m, n, nnz, csrRowPtr, csrColIndex, csrVal, &cfg, nullptr) != SBB_OK)
+    if (!alpha || !beta || m < 0 || n < 0 || nnz < 0 || !csrRowPtr || m > kTiledMaxRows ||
+        (nnz > 0 && (!csrColIndex || !csrVal || !x)) || (m > 0 && !y)) {
+        set_error("bad csr5_kernel arguments");
         return -1;
-    int rc = sbb_spmv(plan, *alpha, x, *beta, y, nullptr);
-    if (rc == SBB_OK) rc = sbb_plan_check(plan);
-    sbb_plan_destroy(plan);
-    return rc == SBB_OK ? 0 : -1;
+    }
+    if (ranges_overlap(x, (size_t)n * 8, y, (size_t)m * 8)) {
+        set_error("x and y overlap (the kernels read x while they write y)");
+        return -1;
+    }
+    const cudaStream_t s = nullptr;
+    Plan p;
+    p.m = m;
+    p.n = n;
+    p.nnz = nnz;
+    p.rowptr = csrRowPtr;
+    p.col = csrColIndex;
+    p.val = csrVal;
+    p.device_runs = true;
+    unsigned *chk = nullptr, h[4] = {};
+    if (dev_malloc_async(reinterpret_cast<void **>(&chk), sizeof(h), s) != cudaSuccess) {
+        set_error("csr5_kernel: device allocation failed");
+        return -1;
+    }
+    cudaMemsetAsync(chk, 0, sizeof(h), s);
+    launch_csr_check(csrRowPtr, m, nnz, csrColIndex, n, chk, reinterpret_cast<int *>(chk + 2), s);
+    cudaMemcpyAsync(h, chk, sizeof(h), cudaMemcpyDeviceToHost, s);
+    cudaError_t e = cudaStreamSynchronize(s);
+    cudaFreeAsync(chk, s);
+    if (e != cudaSuccess || h[0]) {
+        set_error(e != cudaSuccess ? cudaGetErrorString(e)
+                  : h[0] & ST_BAD_ROWPTR ? "row pointer is not monotone within [0, nnz]"
+                                         : "column index out of range [0, n)");
+        return -1;
+    }
+    sbb_config cfg{};
+    once_choice(m, nnz, (int)h[2], &cfg);
+    int rc = plan_build_unchecked(&p, &cfg, s);
+    if (rc == SBB_OK) rc = plan_run(&p, *alpha, x, *beta, y, s);
+    unsigned st = 0;
+    if (rc == SBB_OK) {
+        cudaMemcpyAsync(&st, p.status, sizeof(st), cudaMemcpyDeviceToHost, s);
+        e = cudaStreamSynchronize(s);
+    }
+    plan_free(&p, s);
+    if (rc != SBB_OK) return -1;
+    if (e != cudaSuccess || st) {
+        set_error(e != cudaSuccess ? cudaGetErrorString(e) : "csr5_kernel: device status");
+        return -1;
+    }
+    return 0;
 }
 
 }  // namespace sbb

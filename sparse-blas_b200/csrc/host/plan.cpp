@@ -164,6 +164,22 @@ static bool even_rows(int m, int nnz, int max_row)
     return max_row <= 4 * v;
 }
 
+// The kernel for one product on the caller's arrays, without a copy: vector CSR
+// for even rows, with about a third of the mean row length as lanes (us for 4,
+// 8, 16, 32 lanes: rows of 6 13.0, 17.3, -, -; of 24 -, 18.6, 18.8, 25.5; of 100
+// -, 36.7, 30.9, 30.9), else the merge path (6 items a lane take as long).
+void once_choice(int m, int nnz, int max_row, sbb_config *c)
+{
+    if (even_rows(m, nnz, max_row)) {
+        c->kernel = SBB_KERNEL_VECTOR;
+        c->vector_width = 4;
+        while (c->vector_width < 32 && 3LL * c->vector_width * m < nnz) c->vector_width <<= 1;
+    } else {
+        c->kernel = SBB_KERNEL_MERGE;
+        c->items_per_thread = 8;
+    }
+}
+
 // A validated plan of row slices, `width` lanes a row (0: by the mean row
 // length).  fall_back: 1 instead of an error when the copy does not fit or
 // finds a column out of range, for a caller whose other choice needs no copy

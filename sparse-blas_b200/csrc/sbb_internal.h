@@ -301,6 +301,8 @@ int plan_run(Plan *p, double alpha, const void *x, double beta, double *y,
 void plan_free(Plan *p, cudaStream_t s);
 int default_kernel_choice(int m, int nnz, int max_row, int *vector_width, int *ipt, int *sigma);
 int plan_launches(const Plan *p);
+// The configuration of a plan that runs once.
+void once_choice(int m, int nnz, int max_row, sbb_config *c);
 // Optional timing hooks (set by sbb_spmv_timed for the calling thread): the
 // launchers record them immediately before / after their main kernel.
 struct TimingHooks {
