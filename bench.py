@@ -47,7 +47,7 @@ import numpy as np  # noqa: E402
 
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0}
 KERNEL_TAGS = {1: "vector_kernel", 2: "merge_kernel", 3: "tiled_kernel", 5: "rows_kernel",
-               6: "sliced_kernel"}
+               6: "sliced_kernel", 7: "pieces_spmv_kernel"}
 
 
 def algo_bytes(m, n, nnz):

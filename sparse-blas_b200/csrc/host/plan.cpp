@@ -34,7 +34,8 @@ int plan_launches(const Plan *p)
         extern int rows_launches(const Plan *);
         return rows_launches(p);
     }
-    case SBB_KERNEL_SLICED: return 1;
+    case SBB_KERNEL_SLICED:
+    case SBB_KERNEL_PIECES: return 1;
     default: return 0;
     }
 }
@@ -129,6 +130,7 @@ static int dalloc(T **p, size_t count, cudaStream_t s, size_t *acc)
 extern void tiled_free(Plan *, cudaStream_t);
 extern void rows_free(Plan *, cudaStream_t);
 extern void sliced_free(Plan *, cudaStream_t);
+extern void pieces_free(Plan *, cudaStream_t);
 
 void plan_free(Plan *p, cudaStream_t s)
 {
@@ -139,6 +141,7 @@ void plan_free(Plan *p, cudaStream_t s)
     tiled_free(p, s);
     rows_free(p, s);
     sliced_free(p, s);
+    pieces_free(p, s);
     p->tile_row = p->tile_nnz = nullptr;
     p->carry_val = nullptr;
     p->queue = p->status = nullptr;
@@ -149,6 +152,9 @@ extern int tiled_run(Plan *p, double alpha, const void *x, double beta, double *
                      cudaStream_t s);
 extern int sliced_build(Plan *p, cudaStream_t s);
 extern int sliced_run(Plan *p, double alpha, const void *x, double beta, double *y,
+                      cudaStream_t s);
+extern int pieces_build(Plan *p, cudaStream_t s);
+extern int pieces_run(Plan *p, double alpha, const void *x, double beta, double *y,
                       cudaStream_t s);
 extern int rows_build(Plan *p, cudaStream_t s);
 extern int rows_run(Plan *p, double alpha, const void *x, double beta, double *y,
@@ -263,6 +269,11 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
             rc = build_sliced(p, 0, k == SBB_KERNEL_VECTOR, s);
             if (rc <= 0) return rc;  // built, or an error that the choice below has too
         }
+        // long rows: pieces of rows from 1,024 nnz a row in the mean, where they
+        // pass the tiles (k_pieces.cu); FP64 only
+        if (want_stats && k == SBB_KERNEL_TILED && !p->f32 && !c.vector_width && !c.tile_sigma &&
+            p->nnz / p->m >= 1024)
+            k = SBB_KERNEL_PIECES;
         // FP32 storage: 32 x 8 tiles, which measured fastest for that form
         // (0.130 ms vs 0.166 ms for 32 x 4 on the 5.5M-row matrix)
         if (p->f32) sigma = 8;
@@ -338,6 +349,22 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
             return SBB_ERR_ARG;
         }
         return build_sliced(p, w, false, s);
+    }
+    if (k == SBB_KERNEL_PIECES) {
+        if (!validate) {
+            set_error("row pieces need a validated plan");
+            return SBB_ERR_ARG;
+        }
+        rc = pieces_build(p, s);
+        if (rc != SBB_OK) return rc;
+        unsigned st = 0;
+        SBB_CUDA(cudaMemcpyAsync(&st, p->status, sizeof(st), cudaMemcpyDeviceToHost, s));
+        SBB_CUDA(cudaStreamSynchronize(s));
+        if (st & ST_BAD_COL) {
+            set_error("column index out of range [0, n)");
+            return SBB_ERR_INPUT;
+        }
+        return SBB_OK;
     }
     if (k == SBB_KERNEL_TILED) {
         rc = tiled_build(p, s);
@@ -428,6 +455,8 @@ int plan_run(Plan *p, double alpha, const void *x, double beta, double *y, cudaS
         return rows_run(p, alpha, x, beta, y, s);
     case SBB_KERNEL_SLICED:
         return sliced_run(p, alpha, x, beta, y, s);
+    case SBB_KERNEL_PIECES:
+        return pieces_run(p, alpha, x, beta, y, s);
     default:
         set_error("plan has no kernel");
         return SBB_ERR_ARG;

@@ -290,6 +290,7 @@ struct Plan {
     void *tiled = nullptr;   // K3 tile plan (k_tiled.cu)
     void *rows = nullptr;    // K4 row-block plan (k_rows.cu)
     void *sliced = nullptr;  // K5 row slices (k_sliced.cu)
+    void *pieces = nullptr;  // K6 row pieces (k_pieces.cu)
     size_t scratch_bytes = 0;
     int device = 0;
 };

@@ -10,7 +10,7 @@ import ctypes as C
 from ._lib import Config, PlanInfo, last_error, lib
 
 KERNELS = {"auto": 0, "vector": 1, "merge": 2, "tiled": 3, "learned": 4, "rows": 5,
-           "sliced": 6}
+           "sliced": 6, "pieces": 7}
 
 
 class SbbError(RuntimeError):
