@@ -214,6 +214,21 @@ double csrmv_value(double alpha, double sum, double beta, double y0)
     return beta == 0.0 ? alpha * sum : alpha * sum + beta * y0;
 }
 
+// Free memory as the memory checks see it: what the library's pool holds unused,
+// and, unless that alone is `enough`, what the device has free besides.  Asking
+// the driver for that takes 0.08 ms a call, and up to 11 ms on a host with other
+// processes, which was most of the 0.1 ms before a small call's first copy.
+bool free_memory(double enough, size_t *bytes)
+{
+    const size_t idle = pool_idle_bytes();
+    *bytes = capped_free_bytes(idle);
+    if ((double)*bytes > enough) return true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
+    *bytes = capped_free_bytes(free_b + idle);
+    return true;
+}
+
 // The whole call.  Returns the reference's codes: 0, -1 (bad input, not
 // enough memory, device error), 1 (allocation failure).
 int run(int m, int n, long long nnz, double alpha, const double *val, const long long *rp,
@@ -269,18 +284,11 @@ int run(int m, int n, long long nnz, double alpha, const double *val, const long
     for (auto &p : pieces) saved.push_back({p.row, y[p.row]});
 
     // Memory pre-check as the reference does (0.8 x free memory, v1.cu:106-116).
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return -1;
-    free_b = capped_free_bytes(free_b);
     const int hm = hr1 - hr0 + 1;
     double need = (double)nnz * 12.0 + ((double)m + 1.0) * 12.0 + (double)n * 8.0 + (double)hm * 8.0 +
                   (double)((long long)hm + nnz) / 256.0 * 24.0;
-    if (need / 1e9 > 0.8 * ((double)free_b / 1e9)) {
-        pool_trim();  // memory the pool keeps counts as used until it is given back
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return -1;
-        free_b = capped_free_bytes(free_b);
-        if (need / 1e9 > 0.8 * ((double)free_b / 1e9)) return -1;
-    }
+    size_t free_b = 0;
+    if (!free_memory(need / 0.8, &free_b) || need / 1e9 > 0.8 * ((double)free_b / 1e9)) return -1;
 
     int dev = 0;
     cudaGetDevice(&dev);
@@ -567,9 +575,8 @@ int dropin_v2(int m, int n, long long nnz, double *alpha, double *val, long long
     // one GPU: the calling thread's current device (device 0 unless the
     // caller selected another), as the reference with ngpu = 1 uses device 0
     // nb clamp of v2.cu:43: 0.8 x free memory / 16 B per nnz / q.
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return -1;
-    free_b = capped_free_bytes(free_b);
+    size_t free_b = 0;
+    if (!free_memory((double)nb * 16.0 * q / 0.8 + 16.0 * q, &free_b)) return -1;
     long long cap = (long long)(0.8 * ((double)free_b / 1e9) * 1e9 / 16.0) / q;
     nb = std::min(nb, cap);
     if (nb <= 0) return -1;

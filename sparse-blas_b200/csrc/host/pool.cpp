@@ -86,9 +86,15 @@ cudaMemPool_t device_pool()
 
 }  // namespace
 
-void pool_trim()
+size_t pool_idle_bytes()
 {
-    if (cudaMemPool_t pool = device_pool()) cudaMemPoolTrimTo(pool, 0);
+    cudaMemPool_t pool = device_pool();
+    unsigned long long reserved = 0, used = 0;
+    if (!pool ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return 0;
+    return reserved > used ? (size_t)(reserved - used) : 0;
 }
 
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s)

@@ -36,8 +36,8 @@ inline bool ranges_overlap(const void *a, size_t abytes, const void *b, size_t b
 // Stream-ordered memory from the library's pool on the current device; freed
 // with cudaFreeAsync.
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
-// Gives the pool's unused memory back to the system.
-void pool_trim();
+// Memory that the pool holds and nothing uses.
+size_t pool_idle_bytes();
 // Unique id of the calling thread's current context, or 0 when there is none
 // or the driver cannot tell (cuCtxGetId, CUDA 12.0+).  The driver entry points
 // are fetched through the runtime, so the library does not link libcuda itself.
