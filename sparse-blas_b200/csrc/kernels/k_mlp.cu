@@ -104,10 +104,13 @@ static_assert(kParams == kMlpParams, "parameter blob layout");
 __device__ __forceinline__ float relu(float v) { return v > 0.f ? v : 0.f; }
 
 // A block of 256 threads works on kTile samples at a time, with the
-// parameters and the samples' layers in shared memory.  Rows of 64 are 68
+// parameters and the samples' layers in shared memory.  16 samples a block, twice
+// the blocks, is as fast on 500 samples and slower on 4,000 (22.6 and 16.8 us a
+// step), where the sums over twice the parts cost more.  Rows of 64 are 68
 // floats apart: 16-byte reads of eight consecutive rows then fall into
 // different banks.
 constexpr int MT = 256, kTile = 32, kRow = 68;
+constexpr int kPer = kTile / 16;  // samples of a thread in the 64 x 64 layers
 struct TileMem {
     float mu[F], sd[F], W1[H * F], W2[H * kRow], W3[C * kRow];
     float b1[H], b2[H], b3[C + 2];
@@ -184,32 +187,35 @@ __device__ __forceinline__ void tile_forward(TileMem &T, const float *__restrict
         }
     }
     __syncthreads();
-    {  // layer 2: neurons j, j+16, j+32, j+48 of samples n, n+16
+    {  // layer 2: neurons j, j+16, j+32, j+48 of sample n (and n+16)
         const int j = t % 16, n = t / 16;
-        float z[2][4];
+        float z[kPer][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) z[0][q] = z[1][q] = T.b2[j + 16 * q];
+        for (int i = 0; i < kPer; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) z[i][q] = T.b2[j + 16 * q];
 #pragma unroll 4
         for (int k = 0; k < H; k += 4) {
-            const float4 a0 = ld4(T.h1 + n * kRow + k), a1 = ld4(T.h1 + (n + 16) * kRow + k);
+            float4 a[kPer];
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) a[i] = ld4(T.h1 + (n + 16 * i) * kRow + k);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float4 w = ld4(T.W2 + (j + 16 * q) * kRow + k);
-                z[0][q] = __fmaf_rn(w.x, a0.x, z[0][q]);
-                z[0][q] = __fmaf_rn(w.y, a0.y, z[0][q]);
-                z[0][q] = __fmaf_rn(w.z, a0.z, z[0][q]);
-                z[0][q] = __fmaf_rn(w.w, a0.w, z[0][q]);
-                z[1][q] = __fmaf_rn(w.x, a1.x, z[1][q]);
-                z[1][q] = __fmaf_rn(w.y, a1.y, z[1][q]);
-                z[1][q] = __fmaf_rn(w.z, a1.z, z[1][q]);
-                z[1][q] = __fmaf_rn(w.w, a1.w, z[1][q]);
+#pragma unroll
+                for (int i = 0; i < kPer; ++i) {
+                    z[i][q] = __fmaf_rn(w.x, a[i].x, z[i][q]);
+                    z[i][q] = __fmaf_rn(w.y, a[i].y, z[i][q]);
+                    z[i][q] = __fmaf_rn(w.z, a[i].z, z[i][q]);
+                    z[i][q] = __fmaf_rn(w.w, a[i].w, z[i][q]);
+                }
             }
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            T.h2[n * kRow + j + 16 * q] = n < ns ? relu(z[0][q]) : 0.f;
-            T.h2[(n + 16) * kRow + j + 16 * q] = n + 16 < ns ? relu(z[1][q]) : 0.f;
-        }
+        for (int i = 0; i < kPer; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                T.h2[(n + 16 * i) * kRow + j + 16 * q] = n + 16 * i < ns ? relu(z[i][q]) : 0.f;
     }
     __syncthreads();
     if (t < kTile * C) {  // layer 3: one output of one sample
@@ -249,7 +255,7 @@ mlp_forward_kernel(const float *__restrict__ P, const float *__restrict__ X, int
 // samples took 716 us, 0.6 ms of it in 22 blocks of 4,000-step chains.  Here
 // 125 blocks hold 32 samples each, every stage is a register-tiled product
 // over shared memory, and the sums over blocks are left to
-// mlp_update_kernel: two launches and 21 us a step (12 us for 500 samples), bound by the latency of
+// mlp_update_kernel: two launches and 17 us a step (12 us for 500 samples), bound by the latency of
 // its seven dependent stages (6.3 MFLOP a block).
 constexpr int kPartRow = (kParams + 1 + 31) / 32 * 32;
 __global__ void __launch_bounds__(MT)
@@ -285,6 +291,7 @@ mlp_step_kernel(const float *__restrict__ P, const float *__restrict__ X, int N,
         __syncthreads();
         if (t < C * H / 4) {  // W3: output c, layer-2 neurons 4k ..
             const int c = t / 16, k = t % 16 * 4;
+#pragma unroll 8
             for (int n = 0; n < kTile; ++n) {
                 const float4 a = ld4(T.h2 + n * kRow + k);
                 const float d = T.dy[n * 8 + c];
@@ -317,26 +324,29 @@ mlp_step_kernel(const float *__restrict__ P, const float *__restrict__ X, int N,
 #pragma unroll
                 for (int r = 0; r < 4; ++r) g2[q][r] = __fmaf_rn(dd[q], aa[r], g2[q][r]);
         }
-        // errors of layer 1: neurons 4*tk .. of samples tj and tj + 16
-        float d1[2][4] = {};
+        // errors of layer 1: neurons 4*tk .. of sample tj (and tj + 16)
+        float d1[kPer][4] = {};
 #pragma unroll 4
         for (int j = 0; j < H; j += 4) {
-            const float4 e0 = ld4(T.h2 + tj * kRow + j), e1 = ld4(T.h2 + (tj + 16) * kRow + j);
-            const float f0[4] = {e0.x, e0.y, e0.z, e0.w}, f1[4] = {e1.x, e1.y, e1.z, e1.w};
+            float e[kPer][4];
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) {
+                const float4 v = ld4(T.h2 + (tj + 16 * i) * kRow + j);
+                e[i][0] = v.x, e[i][1] = v.y, e[i][2] = v.z, e[i][3] = v.w;
+            }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float4 w = ld4(T.W2 + (j + q) * kRow + 4 * tk);
                 const float ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    d1[0][r] = __fmaf_rn(ww[r], f0[q], d1[0][r]);
-                    d1[1][r] = __fmaf_rn(ww[r], f1[q], d1[1][r]);
-                }
+                for (int i = 0; i < kPer; ++i)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) d1[i][r] = __fmaf_rn(ww[r], e[i][q], d1[i][r]);
             }
         }
         __syncthreads();  // every thread is done with layer 1's values
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < kPer; ++i)
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 float &h = T.h1[(tj + 16 * i) * kRow + 4 * tk + r];
@@ -345,6 +355,7 @@ mlp_step_kernel(const float *__restrict__ P, const float *__restrict__ X, int N,
         __syncthreads();
         if (t < H * F / 4) {  // W1: neuron j, inputs 4f ..
             const int j = t / 3, f = t % 3 * 4;
+#pragma unroll 8
             for (int n = 0; n < kTile; ++n) {
                 const float4 a = ld4(T.x + n * F + f);
                 const float d = T.h1[n * kRow + j];
@@ -357,8 +368,10 @@ mlp_step_kernel(const float *__restrict__ P, const float *__restrict__ X, int N,
         // biases: b1 by threads 0-63, b2 by 64-127, b3 by 128-133
         if (t < 2 * H) {
             const float *d = (t < H ? T.h1 : T.h2) + t % H;
+#pragma unroll 8
             for (int n = 0; n < kTile; ++n) gb = __fadd_rn(gb, d[n * kRow]);
         } else if (t < 2 * H + C) {
+#pragma unroll 8
             for (int n = 0; n < kTile; ++n) gb = __fadd_rn(gb, T.dy[n * 8 + t - 2 * H]);
         }
     }
