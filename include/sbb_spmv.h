@@ -100,9 +100,11 @@ enum {
                               for short, even rows (vector_width: W = 1, 2, 4,
                               8 or 16, 0 = from mean row length).  No
                               counterpart in the reference. */
-    SBB_KERNEL_PIECES = 7, /* K6: rows in pieces of at most 256 to 1,024 nnz, a
-                              warp each, from the caller's arrays (no copy); for
-                              long rows.  No counterpart in the reference. */
+    SBB_KERNEL_PIECES = 7, /* K6: rows in pieces of at most 64 to 1,024 nnz,
+                              vector_width (8 or 32, 0 = 32) lanes each, from
+                              the caller's arrays (no copy); for long rows and
+                              small matrices.  No counterpart in the
+                              reference. */
     SBB_KERNEL_ROWS = 5    /* K4: blocks of <= 32 rows and <= 384 nnz (rows
                               longer than 384 nnz split into pieces), staged
                               into shared memory by TMA straight from the

@@ -260,7 +260,7 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
         if (c.kernel == SBB_KERNEL_TILED && p->m > kTiledMaxRows)
             c = batch_class_config(kBatchMergeClass);
     }
-    int vw = 0, ipt = 0, sigma = 0;
+    int vw = 0, ipt = 0, sigma = 0, piece_width = 32;
     int k = c.kernel;
     if (k == SBB_KERNEL_AUTO) {
         k = default_kernel_choice(p->m, p->nnz, want_stats ? p->max_row : INT_MAX, &vw, &ipt, &sigma);
@@ -269,11 +269,20 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
             rc = build_sliced(p, 0, k == SBB_KERNEL_VECTOR, s);
             if (rc <= 0) return rc;  // built, or an error that the choice below has too
         }
-        // long rows: pieces of rows from 1,024 nnz a row in the mean, where they
-        // pass the tiles (k_pieces.cu); FP64 only
-        if (want_stats && k == SBB_KERNEL_TILED && !p->f32 && !c.vector_width && !c.tile_sigma &&
-            p->nnz / p->m >= 1024)
-            k = SBB_KERNEL_PIECES;
+        // Row pieces (k_pieces.cu) pass the tiles on long rows, FP64, from 1,024 nnz
+        // a row in the mean, with 32 lanes a piece; and with 8 lanes a piece in calls
+        // on small matrices, where they need one launch and the tiles two (us a call
+        // from a program and on the device alone: 65k nnz 10.2 and 4.8 with tiles, 8.0
+        // and 5.2 with pieces; FP32 storage 10.4 and 8.4, 8.0 and 5.6; from 200k nnz
+        // the device's time decides: 215k nnz 5.0 and 6.1).
+        if (want_stats && k == SBB_KERNEL_TILED && !p->lane32 && !c.vector_width && !c.tile_sigma) {
+            if (p->nnz <= 1 << 17) {
+                k = SBB_KERNEL_PIECES;
+                piece_width = 8;
+            } else if (!p->f32 && p->nnz / p->m >= 1024) {
+                k = SBB_KERNEL_PIECES;
+            }
+        }
         // FP32 storage: 32 x 8 tiles, which measured fastest for that form
         // (0.130 ms vs 0.166 ms for 32 x 4 on the 5.5M-row matrix)
         if (p->f32) sigma = 8;
@@ -351,8 +360,9 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
         return build_sliced(p, w, false, s);
     }
     if (k == SBB_KERNEL_PIECES) {
-        if (!validate) {
-            set_error("row pieces need a validated plan");
+        if (!c.vector_width) p->vector_width = vw = piece_width;
+        if (!validate || (vw != 8 && vw != 32)) {
+            set_error("row pieces need a validated plan and vector_width 8 or 32");
             return SBB_ERR_ARG;
         }
         rc = pieces_build(p, s);
