@@ -12,7 +12,7 @@
 //
 // Why: on such rows the tiles' instructions (217 a 128-nnz tile) and L1 traffic
 // (76 % of its data pipe) come before HBM, and every tile carries its row on; here
-// 32 nnz take about 14 instructions.  FP64, against 32 x 4 tiles and their fix-up
+// 32 nnz take 29 instructions in all (tiles 51).  FP64, against 32 x 4 tiles and their fix-up
 // (us): 4,284 rows of 2,770 in the mean 28.4 vs 32.1, 20,000 of 2,670 114 vs 124
 // (5.6 TB/s), 2,000 of 1,590 12.9 vs 14.4, 20,000 of 1,020 52.9 vs 53.0; rows of
 // 310 17.0 vs 14.8, and with FP32 storage no difference, so both keep the tiles.

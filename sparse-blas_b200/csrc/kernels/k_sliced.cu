@@ -13,8 +13,8 @@
 // Why: the vector kernel reads the caller's arrays with V lanes a row, and on
 // short rows its issue slots (61 % used; 128 warp instructions per 24-nnz row,
 // most of them in the butterflies and the ragged ends of each row) and
-// latency come before HBM (24 %).  Here a step of 32 nnz takes about 16
-// instructions.  Measured against it (FP64, beta = 0.5; us): 200k rows of 24
+// latency come before HBM (24 %).  Here 32 nnz take 40 instructions in
+// all, 128 there.  Measured against it (FP64, beta = 0.5; us): 200k rows of 24
 // nnz in a band 13.6 vs 26.7; 500k rows of 6 10.6 vs 19.1; 100k rows of 50 in
 // diagonal blocks 14.4 vs 21.5; 1M rows of 40 in a band 91.6 vs 136.5 (5.5 TB/s);
 // 700k rows of 0 to 8, half of them empty, 12.0 vs 16.3; FP32 storage, 200k
