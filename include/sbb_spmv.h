@@ -116,7 +116,8 @@ enum {
 
 typedef struct {
     int kernel;            /* SBB_KERNEL_*                                  */
-    int vector_width;      /* K1: 2,4,8,16,32 (0 = from mean row length)    */
+    int vector_width;      /* lanes per row or piece: K1 2,4,8,16,32, K5 1,2,4,
+                              8,16, K6 8,32 (0 = from mean row length)      */
     int items_per_thread;  /* K2: merge items per thread (0 = default)      */
     int persistent;        /* K2: >0 = persistent CTAs per SM with a device
                               work queue; 0 = one CTA per tile              */

@@ -99,7 +99,11 @@ size_t pool_idle_bytes()
 
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s)
 {
-    cudaMemPool_t pool = device_pool();
+    // In a stream capture the allocation becomes a node of the graph, from the
+    // default pool; making a pool is not allowed there.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) cudaGetLastError();
+    cudaMemPool_t pool = capturing == cudaStreamCaptureStatusNone ? device_pool() : nullptr;
     if (!pool) return cudaMallocAsync(p, bytes, s);
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
     if (e == cudaErrorMemoryAllocation) {

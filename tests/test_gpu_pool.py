@@ -56,3 +56,39 @@ def test_pool_bounded_and_threads(cuda):
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     assert free0 - torch.cuda.mem_get_info(0)[0] <= total // 32 + (1 << 30)
+
+
+CAPTURE = """
+import ctypes as C, sys
+sys.path.insert(0, sys.argv[1])
+import torch
+from sbb import lib
+rp = torch.tensor([0, 2, 5], dtype=torch.int32, device="cuda")
+col = torch.arange(5, dtype=torch.int32, device="cuda")
+out, ref = (torch.zeros(12, device="cuda") for _ in range(2))
+def call(t, s):
+    return lib().sbb_features(2, 5, 5, C.c_void_p(rp.data_ptr()), C.c_void_p(col.data_ptr()),
+                              C.c_void_p(t.data_ptr()), C.c_void_p(s.cuda_stream))
+s = torch.cuda.Stream()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=s):  # the library's first allocation
+    assert call(out, torch.cuda.current_stream()) == 0
+g.replay()
+torch.cuda.synchronize()
+assert call(ref, torch.cuda.current_stream()) == 0
+torch.cuda.synchronize()
+assert torch.equal(out, ref) and float(ref.abs().sum()) > 0
+"""
+
+
+def test_first_allocation_inside_a_capture(cuda):
+    """A call that allocates stream-ordered scratch, captured in a graph before
+    the library has made its pool (in a process of its own)."""
+    import os
+    import subprocess
+    import sys
+    import sbb
+    pkg = os.path.dirname(os.path.dirname(os.path.abspath(sbb.__file__)))
+    r = subprocess.run([sys.executable, "-c", CAPTURE, pkg], capture_output=True, text=True,
+                       timeout=120)
+    assert r.returncode == 0, r.stderr[-800:]
