@@ -127,7 +127,7 @@ void launch_merge_t(const CsrView &A, const MergeScratch &S, double alpha,
 {
     const auto *val = static_cast<const typename PT::V *>(A.val);
     if (S.tiles > 0) {
-        const auto kern = merge_kernel<PT, ACC, IPT>;
+        constexpr auto kern = merge_kernel<PT, ACC, IPT>;
         long long blocks = (S.tiles + WPB - 1) / WPB;
         const bool queued = S.queue && S.persistent_ctas > 0 && S.persistent_ctas < blocks;
         int item = S.queue_item > 0 ? S.queue_item : 1;
@@ -135,7 +135,7 @@ void launch_merge_t(const CsrView &A, const MergeScratch &S, double alpha,
             // kMergeGroup segments a warp when that still makes eight waves of
             // blocks, else fewer, so that the last wave stays small (us for 4, 2
             // and 1: 7.6M nnz 49.2, 45.0, 43.1; 60M nnz 282, -, 343)
-            const LaunchShape ls = cached_launch_shape(kern, NT, 0);
+            const LaunchShape ls = cached_launch_shape<kern>(NT, 0);
             item = kMergeGroup;
             while (item > 1 && blocks < 8LL * item * ls.sms * ls.occ) item >>= 1;
             blocks = (S.tiles + (long long)item * WPB - 1) / ((long long)item * WPB);

@@ -421,9 +421,9 @@ void launch_rows_n(const RowsPlan &R, const Plan *p, double alpha, const typenam
                    double beta, double *y, cudaStream_t s)
 {
     using V = typename PT::V;
-    auto kern = rows_kernel<PT, NMAX, MINB>;
+    constexpr auto kern = rows_kernel<PT, NMAX, MINB>;
     constexpr size_t smem = (size_t)RW * kNbuf * RowsSlot<V, NMAX>::BYTES;
-    const LaunchShape ls = cached_launch_shape(kern, RW * 32, smem);
+    const LaunchShape ls = cached_launch_shape<kern>(RW * 32, smem);
     const long long want = (R.nblk + RW - 1) / RW;
     const long long cap = (long long)ls.sms * ls.occ;
     const int grid = (int)(want < cap ? want : cap);

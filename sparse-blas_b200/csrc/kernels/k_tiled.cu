@@ -396,10 +396,10 @@ void launch_tiled_n(const TiledPlan &T, int m, int n, long long nnz, double alph
                     const typename PT::V *x, double beta, double *y, unsigned *status,
                     cudaStream_t s)
 {
-    auto kern = tiled_kernel<PT, ACC, SIGMA, 2, NE>;
+    constexpr auto kern = tiled_kernel<PT, ACC, SIGMA, 2, NE>;
     constexpr size_t smem =
         (size_t)TW * (2 * tile_bytes_of(SIGMA, sizeof(typename PT::V)) + sum_bytes_of(SIGMA));
-    const LaunchShape ls = cached_launch_shape(kern, TW * 32, smem);
+    const LaunchShape ls = cached_launch_shape<kern>(TW * 32, smem);
     long long want = (T.tiles + TW - 1) / TW;
     long long cap = (long long)ls.sms * ls.occ;
     int grid = (int)(want < cap ? want : cap);

@@ -39,8 +39,8 @@ template <typename PT, typename ACC, int V>
 void launch_vector_v(const CsrView &A, double alpha, const typename PT::V *x, double beta,
                      double *y, unsigned *status, cudaStream_t s)
 {
-    const auto kern = vector_kernel<PT, ACC, V>;
-    const LaunchShape ls = cached_launch_shape(kern, VT, 0);
+    constexpr auto kern = vector_kernel<PT, ACC, V>;
+    const LaunchShape ls = cached_launch_shape<kern>(VT, 0);
     // Shares of a few chunks: enough for the prefetches to run ahead, small
     // enough that the warps end together.
     const long long warps = (long long)ls.sms * ls.occ * (VT / 32);
