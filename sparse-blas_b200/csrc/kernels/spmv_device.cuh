@@ -6,6 +6,7 @@
 
 #include "../sbb_internal.h"
 #include "common.cuh"
+#include "lane_index.cuh"
 
 namespace sbb {
 
@@ -94,18 +95,16 @@ __device__ __forceinline__ void vector_rows(int r0, int count, int n,
         const bool in = lane < min(CR, count - at);
         if (in && beta != 0.0) yv = ld_y(y + r0 + at + lane, stream);
         if (at + CR < count) prefetch(nlo, nhi);
-        // nnz indices are unsigned: with nnz up to 2^31 - 1 a lane's index runs
-        // to at most nnz - 1 + V (< 2^32), past the int range but never wrapping
-        unsigned k[U], end[U];
+        unsigned k[U], reach[U];
         ACC acc[U];
-        bool any = false;
+        unsigned most = 0;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int q = u * RPW + g;
             k[u] = (unsigned)__shfl_sync(0xffffffffu, lo, q) + (unsigned)li;
-            end[u] = (unsigned)__shfl_sync(0xffffffffu, hi, q);
+            reach[u] = lane_reach(k[u], (unsigned)__shfl_sync(0xffffffffu, hi, q));
             acc[u].zero();
-            any |= k[u] < end[u];
+            most = max(most, reach[u]);
         }
         lo = nlo;
         hi = nhi;
@@ -114,26 +113,24 @@ __device__ __forceinline__ void vector_rows(int r0, int count, int n,
         T v[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            c[u] = ld_stream_if(col + k[u], k[u] < end[u]);
-            v[u] = ld_stream_if(val + k[u], k[u] < end[u]);
+            c[u] = ld_stream_if(col + k[u], 0u < reach[u]);
+            v[u] = ld_stream_if(val + k[u], 0u < reach[u]);
         }
-        while (any) {
+#pragma unroll 1
+        for (unsigned off = 0; off < most; off += V) {
             T xv[U], vn[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) xv[u] = gather_x_if(x, c[u], n, k[u] < end[u], bad);
-            any = false;
+            for (int u = 0; u < U; ++u) xv[u] = gather_x_if(x, c[u], n, off < reach[u], bad);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const unsigned kn = k[u] + V;
-                any |= kn < end[u];
-                c[u] = ld_stream_if(col + kn, kn < end[u]);
-                vn[u] = ld_stream_if(val + kn, kn < end[u]);
+                const bool p = off + V < reach[u];
+                c[u] = ld_stream_if(col + (k[u] + V + off), p);
+                vn[u] = ld_stream_if(val + (k[u] + V + off), p);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                if (k[u] < end[u]) acc[u].mac(v[u], xv[u]);
+                if (off < reach[u]) acc[u].mac(v[u], xv[u]);
                 v[u] = vn[u];
-                k[u] += V;
             }
         }
         double part[U];

@@ -1,0 +1,38 @@
+// The walk of a lane over rows, at the limits of nnz (2^31 - 1), as the vector
+// kernel does it (lane_index.cuh), on the host.
+#include <cstdio>
+#include <initializer_list>
+
+#include "lane_index.cuh"
+
+using sbb::lane_reach;
+
+static int failures = 0;
+static void check(bool ok, const char *what, unsigned a, unsigned b)
+{
+    if (ok) return;
+    failures++;
+    std::printf("failed: %s (%u, %u)\n", what, a, b);
+}
+
+int main()
+{
+    const unsigned last = 0x7fffffffu;  // the largest nnz
+    // A row that is empty (or has one nnz) and starts behind one of `len` nnz, the
+    // two walked together by `v` lanes: first and last steps of the walk.
+    for (unsigned v = 2; v <= 32; v *= 2)
+        for (unsigned len : {last, last - 1, last - 40, 1u << 30})
+            for (unsigned li = 0; li < v; li++)
+                for (unsigned own = 0; own <= 1; own++) {
+                    const unsigned reach = lane_reach(last - own + li, last);
+                    const unsigned most = lane_reach(li, len);
+                    check(reach == (own && li == 0), "nnz of the short row", reach, li);
+                    check(most == len - li, "nnz of the long row", most, li);
+                    unsigned long long off = (most - 1) / v * (unsigned long long)v;
+                    check(off < most && off + v >= most, "last step", most, v);
+                    for (int i = 0; i < 3; i++, off += v)  // it, and two more loaded ahead
+                        check(off <= 0xffffffffull && (unsigned)off >= reach, "walks again", li, v);
+                }
+    if (!failures) std::printf("ok\n");
+    return failures != 0;
+}
