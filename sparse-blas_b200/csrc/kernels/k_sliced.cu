@@ -25,6 +25,7 @@
 
 #include "../sbb_internal.h"
 #include "common.cuh"
+#include "lane_index.cuh"
 
 namespace sbb {
 
@@ -58,7 +59,8 @@ struct SlicedPlan {
 struct SliceLane {
     int row;
     unsigned base, total;
-    int start, len, mine, steps, full;
+    int start, len;
+    unsigned mine, steps, full;
 };
 template <int W>
 __device__ __forceinline__ SliceLane slice_lane(int s, int m, const int *__restrict__ rowptr)
@@ -78,7 +80,7 @@ __device__ __forceinline__ SliceLane slice_lane(int s, int m, const int *__restr
     }
     L.base = (unsigned)__shfl_sync(0xffffffffu, L.start, 0);
     L.total = __reduce_add_sync(0xffffffffu, sub == 0 ? (unsigned)L.len : 0u);
-    L.mine = L.len > sub ? (L.len - sub + W - 1) / W : 0;
+    L.mine = lane_share((unsigned)L.len, sub, W);
     L.steps = __reduce_max_sync(0xffffffffu, L.mine);
     L.full = __reduce_min_sync(0xffffffffu, L.mine);
     return L;
@@ -108,7 +110,7 @@ sliced_kernel(int m, int slices, const int *__restrict__ rowptr, const int *__re
     // steps of all 32 lanes: no predicates, constant offsets
     const int *cp = col + L.base + lane;
     const V *vp = val + L.base + lane;
-    int j = 0;
+    unsigned j = 0;  // a row has up to 2^31 - 1 steps: j runs past int
 #pragma unroll 1
     for (; j + kSteps <= L.full; j += kSteps) {
         int c[kSteps];
@@ -125,7 +127,7 @@ sliced_kernel(int m, int slices, const int *__restrict__ rowptr, const int *__re
         cp += 32 * kSteps;
         vp += 32 * kSteps;
     }
-    unsigned at = L.base + 32u * (unsigned)j;
+    unsigned at = L.base + 32u * j;
     const unsigned before = (1u << lane) - 1u;
 #pragma unroll 1
     for (; j < L.steps; j += kSteps) {
@@ -185,11 +187,11 @@ slice_fill_kernel(const int *__restrict__ rowptr, int m, int n, int slices,
     }
     unsigned at = L.base;
     const unsigned before = (1u << lane) - 1u;
-    for (int j = 0; j < L.steps; ++j) {
+    for (unsigned j = 0; j < L.steps; ++j) {
         const bool p = j < L.mine;
         const unsigned who = __ballot_sync(0xffffffffu, p);
         if (p) {
-            const unsigned from = (unsigned)L.start + (unsigned)(j * W + lane % W);
+            const unsigned from = (unsigned)L.start + j * W + lane % W;
             int c;
             V v;
             if (staged) {

@@ -17,4 +17,10 @@ namespace sbb {
 // a short row wrapped to 0 beside a row of nearly 2^31 nnz, and its walk began again.)
 SBB_HD unsigned lane_reach(unsigned k, unsigned end) { return k < end ? end - k : 0u; }
 
+// How many of a row's `len` nnz lane `sub` of `width` takes: sub, sub + width, ...
+SBB_HD unsigned lane_share(unsigned len, unsigned sub, unsigned width)
+{
+    return len > sub ? (len - sub + width - 1u) / width : 0u;
+}
+
 }  // namespace sbb

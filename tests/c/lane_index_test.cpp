@@ -1,11 +1,12 @@
 // The walk of a lane over rows, at the limits of nnz (2^31 - 1), as the vector
-// kernel does it (lane_index.cuh), on the host.
+// kernel and the row slices do it (lane_index.cuh), on the host.
 #include <cstdio>
 #include <initializer_list>
 
 #include "lane_index.cuh"
 
 using sbb::lane_reach;
+using sbb::lane_share;
 
 static int failures = 0;
 static void check(bool ok, const char *what, unsigned a, unsigned b)
@@ -33,6 +34,17 @@ int main()
                     for (int i = 0; i < 3; i++, off += v)  // it, and two more loaded ahead
                         check(off <= 0xffffffffull && (unsigned)off >= reach, "walks again", li, v);
                 }
+    // Shares of the row slices: together the whole row, evenly.
+    for (unsigned w = 1; w <= 16; w *= 2)
+        for (unsigned len : {0u, 1u, w - 1, w, w + 1, 1000u, last - 16, last - 1, last}) {
+            unsigned long long sum = 0;
+            for (unsigned sub = 0; sub < w; sub++) {
+                const unsigned n = lane_share(len, sub, w);
+                check(n <= len / w + 1 && n >= len / w, "share", len, sub);
+                sum += n;
+            }
+            check(sum == len, "shares of a row", len, w);
+        }
     if (!failures) std::printf("ok\n");
     return failures != 0;
 }
