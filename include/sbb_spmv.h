@@ -338,7 +338,8 @@ int sbb_last_call_phases(double *ms, int n);
  * production use.
  *   SBB_TEST_RESET        disarm every hook (value ignored);
  *   SBB_TEST_FAIL_ALLOC   value = k >= 1: the k-th device allocation the
- *                         library makes from now on fails, once (0 disarms);
+ *                         library makes from now on asks for 2^50 bytes and
+ *                         so fails, once (0 disarms);
  *   SBB_TEST_FREE_BYTES   value >= 0: the drop-in memory pre-check sees at
  *                         most this many free bytes (< 0 disarms);
  *   SBB_TEST_WAIT_BUDGET  value >= 0: in tiled-kernel launches the first wait

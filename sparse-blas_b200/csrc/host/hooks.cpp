@@ -24,9 +24,9 @@ cudaError_t dev_malloc_async(void **p, size_t bytes, cudaStream_t s)
     long long k = g_fail_alloc.load();
     while (k > 0 && !g_fail_alloc.compare_exchange_weak(k, k - 1)) {
     }
-    if (k == 1) {  // this is the armed allocation
+    if (k == 1) {  // this is the armed allocation: more than any device has
         *p = nullptr;
-        return cudaErrorMemoryAllocation;
+        bytes = (size_t)1 << 50;
     }
     return pool_malloc_async(p, bytes, s);
 }

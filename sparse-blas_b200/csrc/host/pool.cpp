@@ -104,13 +104,15 @@ cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s)
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) cudaGetLastError();
     cudaMemPool_t pool = capturing == cudaStreamCaptureStatusNone ? device_pool() : nullptr;
-    if (!pool) return cudaMallocAsync(p, bytes, s);
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+    if (pool && e == cudaErrorMemoryAllocation) {
         cudaMemPoolTrimTo(pool, 0);
+        cudaGetLastError();
         e = cudaMallocFromPoolAsync(p, bytes, pool, s);
     }
+    // The caller gets the code and may go on without this memory: it must not
+    // meet the same error again behind its next launch.
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
     return e;
 }
 
