@@ -62,6 +62,7 @@ static void batch_free(sbb_batch_s *b)
         plan_free(p, nullptr);
         delete p;
     }
+    pool_settle(nullptr);
     delete b;
 }
 
@@ -471,6 +472,7 @@ int sbb_tune_classes(int m, int n, int nnz, const int *d_rowptr, const int *d_co
         }
         plan_free(&p, s);
     }
+    pool_settle(s);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     return rc;

@@ -659,7 +659,8 @@ double min_free_gb(int ngpu)
     for (int d = 0; d < upto; d++) {
         size_t f = 0, t = 0;
         cudaSetDevice(d);
-        if (cudaMemGetInfo(&f, &t) == cudaSuccess) best = std::min(best, (double)f / 1e9);
+        const size_t idle = pool_trim();  // what the library keeps between calls is free too
+        if (cudaMemGetInfo(&f, &t) == cudaSuccess) best = std::min(best, (double)(f + idle) / 1e9);
     }
     cudaSetDevice(prev);
     return best;
@@ -719,6 +720,7 @@ int csr5_entry(int m, int n, int nnz, double *alpha, double *csrVal, int *csrRow
         e = cudaStreamSynchronize(s);
     }
     plan_free(&p, s);
+    pool_settle(s);
     if (rc != SBB_OK) return -1;
     if (e != cudaSuccess || st) {
         set_error(e != cudaSuccess ? cudaGetErrorString(e) : "csr5_kernel: device status");

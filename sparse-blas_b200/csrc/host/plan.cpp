@@ -651,6 +651,7 @@ int sbb_plan_destroy(sbb_plan_t plan)
     cudaSetDevice(plan->p.device);
     cudaDeviceSynchronize();  // products in flight on any stream
     plan_free(&plan->p, nullptr);
+    pool_settle(nullptr);
     delete plan;
     return SBB_OK;
 }

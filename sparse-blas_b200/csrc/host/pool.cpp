@@ -7,9 +7,13 @@
 // took 2.6 to 10 ms a call for 0.25 ms of kernels.  The library therefore has
 // a pool of its own on each device, which keeps at most 1/32 of the device's
 // memory while nothing uses it, gives all of that back when an allocation of
-// the library does not fit, and leaves the default pool and its settings to
-// the program.  Stream order makes it safe for several streams; the driver
-// makes it safe for several threads.
+// the library does not fit or the program asks for the free memory
+// (get_gpu_availble_mem), and leaves the default pool and its settings to
+// the program.  A pool gives back what it holds above its bound at the next
+// synchronisation, so what frees large buffers ends with pool_settle, which
+// synchronises once more if that is needed (each time would cost a one-off
+// product 4 us of 107).  Stream order makes the pool safe for several streams;
+// the driver makes it safe for several threads.
 #include <cuda.h>  // driver types only; the entry points are fetched at run time
 #include <cuda_runtime.h>
 
@@ -53,8 +57,9 @@ struct DevicePool {
 
 // The current device's pool, made the first time and again when the device's
 // context has been replaced (after cudaDeviceReset, for example); null when
-// there is none to be had, and the default pool serves.
-cudaMemPool_t device_pool()
+// there is none to be had, and the default pool serves, or with make == false
+// when there is none yet.
+cudaMemPool_t device_pool(bool make = true)
 {
     static std::mutex mu;
     static DevicePool pools[64];
@@ -64,6 +69,7 @@ cudaMemPool_t device_pool()
     DevicePool &d = pools[dev];
     unsigned long long ctx = current_context_id();
     if (d.pool && ctx != 0 && d.ctx == ctx) return d.pool;
+    if (!make) return nullptr;
     size_t free_b = 0, total_b = 0;  // also makes the device's context current
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return nullptr;
     ctx = current_context_id();
@@ -86,15 +92,37 @@ cudaMemPool_t device_pool()
 
 }  // namespace
 
+static bool pool_bytes(cudaMemPool_t pool, unsigned long long *reserved, unsigned long long *used)
+{
+    return pool &&
+           cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, reserved) == cudaSuccess &&
+           cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, used) == cudaSuccess;
+}
+
 size_t pool_idle_bytes()
 {
-    cudaMemPool_t pool = device_pool();
     unsigned long long reserved = 0, used = 0;
-    if (!pool ||
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
-        return 0;
+    if (!pool_bytes(device_pool(), &reserved, &used)) return 0;
     return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+void pool_settle(cudaStream_t s)
+{
+    cudaMemPool_t pool = device_pool(false);
+    unsigned long long reserved = 0, used = 0, keep = 0;
+    if (pool_bytes(pool, &reserved, &used) && reserved > used &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
+        reserved > keep)
+        cudaStreamSynchronize(s);
+}
+
+size_t pool_trim()
+{
+    cudaMemPool_t pool = device_pool(false);
+    unsigned long long reserved = 0, used = 0;
+    if (!pool) return 0;
+    cudaMemPoolTrimTo(pool, 0);
+    return pool_bytes(pool, &reserved, &used) && reserved > used ? (size_t)(reserved - used) : 0;
 }
 
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s)

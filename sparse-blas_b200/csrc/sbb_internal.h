@@ -38,6 +38,12 @@ inline bool ranges_overlap(const void *a, size_t abytes, const void *b, size_t b
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
 // Memory that the pool holds and nothing uses.
 size_t pool_idle_bytes();
+// After the frees that end a plan or a call, enqueued on s: when the pool holds
+// more than its bound, waits for them, and the excess goes back to the device.
+void pool_settle(cudaStream_t s);
+// Gives what the current device's pool holds unused back to the device; returns
+// the bytes of it whose frees have yet to be synchronised with.
+size_t pool_trim();
 // Unique id of the calling thread's current context, or 0 when there is none
 // or the driver cannot tell (cuCtxGetId, CUDA 12.0+).  The driver entry points
 // are fetched through the runtime, so the library does not link libcuda itself.
