@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "../sbb_internal.h"
+#include "context_table.h"
 
 namespace sbb {
 
@@ -50,30 +51,25 @@ unsigned long long current_context_id()
 
 namespace {
 
-struct DevicePool {
-    cudaMemPool_t pool = nullptr;
-    unsigned long long ctx = 0;  // identity of the context the pool belongs to
-};
-
-// The current device's pool, made the first time and again when the device's
-// context has been replaced (after cudaDeviceReset, for example); null when
-// there is none to be had, and the default pool serves, or with make == false
-// when there is none yet.
+// The pool of the current device's current context, made the first time; null
+// when there is none to be had, and the default pool serves, or with make ==
+// false when there is none yet.  (After cudaDeviceReset the context is another.)
 cudaMemPool_t device_pool(bool make = true)
 {
     static std::mutex mu;
-    static DevicePool pools[64];
+    static auto &pools = *new ContextTable<cudaMemPool_t>;  // outlives static destructors
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
-    DevicePool &d = pools[dev];
     unsigned long long ctx = current_context_id();
-    if (d.pool && ctx != 0 && d.ctx == ctx) return d.pool;
+    if (ctx != 0)
+        if (cudaMemPool_t *known = pools.find(dev, ctx)) return *known;
     if (!make) return nullptr;
     size_t free_b = 0, total_b = 0;  // also makes the device's context current
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return nullptr;
     ctx = current_context_id();
     if (ctx == 0) return nullptr;
+    if (cudaMemPool_t *known = pools.find(dev, ctx)) return *known;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -85,8 +81,7 @@ cudaMemPool_t device_pool(bool make = true)
     }
     unsigned long long keep = total_b / 32;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    d.pool = pool;
-    d.ctx = ctx;
+    pools.add(dev, ctx, pool);
     return pool;
 }
 
