@@ -270,13 +270,15 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
             if (rc <= 0) return rc;  // built, or an error that the choice below has too
         }
         // Row pieces (k_pieces.cu) pass the tiles on long rows, FP64, from 1,024 nnz
-        // a row in the mean, with 32 lanes a piece; and with 8 lanes a piece in calls
-        // on small matrices, where they need one launch and the tiles two (us a call
-        // from a program and on the device alone: 65k nnz 10.2 and 4.8 with tiles, 8.0
-        // and 5.2 with pieces; FP32 storage 10.4 and 8.4, 8.0 and 5.6; from 200k nnz
-        // the device's time decides: 215k nnz 5.0 and 6.1).
+        // a row in the mean, with 32 lanes a piece; and with 8 lanes a piece on small
+        // matrices, where they need one launch and the tiles two (us a call from a
+        // program: 63k power-law nnz 10.0 with tiles, 8.0 with pieces; from 200k nnz the
+        // device's time decides: 215k nnz 5.0 and 6.1).  Small in rows as well: every
+        // row, empty ones too, is a piece that a lane group looks at (100k nnz, us on
+        // the device: 30,000 rows 8.9 with tiles, 5.7 with pieces; 50,000 5.6 and 8.1;
+        // 100,000 8.9 and 10.6; 1M 9.1 and 37.9).
         if (want_stats && k == SBB_KERNEL_TILED && !p->lane32 && !c.vector_width && !c.tile_sigma) {
-            if (p->nnz <= 1 << 17) {
+            if (p->nnz <= 1 << 17 && p->m <= 1 << 15) {
                 k = SBB_KERNEL_PIECES;
                 piece_width = 8;
             } else if (!p->f32 && p->nnz / p->m >= 1024) {
