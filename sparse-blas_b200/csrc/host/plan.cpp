@@ -271,16 +271,18 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
         }
         // Row pieces (k_pieces.cu) pass the tiles on long rows, FP64, from 1,024 nnz
         // a row in the mean, with 32 lanes a piece; and with 8 lanes a piece on small
-        // matrices, where they need one launch and the tiles two (us a call from a
-        // program: 63k power-law nnz 10.0 with tiles, 8.0 with pieces; from 200k nnz the
-        // device's time decides: 215k nnz 5.0 and 6.1).  Small in rows as well: every
+        // matrices, where they need one launch and the tiles two (63k power-law nnz, us a
+        // call from a program and on the device alone: 10.0 and 4.7 with tiles, 8.0 and
+        // 4.7 with pieces; from 200k nnz the device's time decides: 215k nnz 5.0 and
+        // 6.1), with 32 there too from 512 nnz a row (100 x 1,000 nnz 4.5 and one row of
+        // 131,072 5.3; tiles 4.6 and 6.4).  Small in rows as well: every
         // row, empty ones too, is a piece that a lane group looks at (100k nnz, us on
         // the device: 30,000 rows 8.9 with tiles, 5.7 with pieces; 50,000 5.6 and 8.1;
         // 100,000 8.9 and 10.6; 1M 9.1 and 37.9).
         if (want_stats && k == SBB_KERNEL_TILED && !p->lane32 && !c.vector_width && !c.tile_sigma) {
             if (p->nnz <= 1 << 17 && p->m <= 1 << 15) {
                 k = SBB_KERNEL_PIECES;
-                piece_width = 8;
+                piece_width = p->nnz / std::max(p->m, 1) >= 512 ? 32 : 8;
             } else if (!p->f32 && p->nnz / p->m >= 1024) {
                 k = SBB_KERNEL_PIECES;
             }

@@ -1,23 +1,33 @@
-// k_pieces.cu — K6: rows in pieces: long rows in pieces of at most 256 to 1,024
-// nnz, a warp each, and the rows of small matrices in pieces of at most 64, eight
-// lanes each (FP64 and FP32-storage forms).
+// k_pieces.cu — K6: rows in pieces: long rows in pieces of 256 to 2,048 nnz, a
+// warp each, and the rows of small matrices in pieces of 64, eight lanes each
+// (larger ones where a row would have more than 2,048 or 1,024 pieces).  FP64 and
+// FP32-storage forms.
 //
 // A group of 32 lanes (or 8, with 8 for 32 in what follows) reads its piece
 // straight from the caller's arrays, 32 nnz a step on 32-nnz boundaries; each lane
-// sums its own nnz and the group's sums meet in one butterfly at the end.  A row of one piece is written at once.  A row of several
-// keeps one partial sum per piece; the group that finishes last (an atomic count
-// per row that wraps to 0 by itself) adds them in piece order, so the result does
-// not depend on which that was, and no second kernel is needed.  The plan is
-// the list of pieces, 28 bytes each, and no copy of the matrix.
+// sums its own nnz and the group's sums meet in one butterfly at the end.  A row of
+// one piece is written at once.  A row of several keeps one partial sum per piece;
+// the warp with the piece that finishes last (an atomic count per row that wraps to
+// 0 by itself) adds them in piece order, so the result does not depend on which
+// that was, and no second kernel is needed.  The plan is the list of pieces, 28
+// bytes each, and no copy of the matrix.
 //
-// Why: on such rows the tiles' instructions (217 a 128-nnz tile) and L1 traffic
+// Why: on long rows the tiles' instructions (217 a 128-nnz tile) and L1 traffic
 // (76 % of its data pipe) come before HBM, and every tile carries its row on; here
-// 32 nnz take 29 instructions in all (tiles 51).  FP64, against 32 x 4 tiles and their fix-up
-// (us): 4,284 rows of 2,770 in the mean 28.4 vs 32.1, 20,000 of 2,670 114 vs 124
-// (5.6 TB/s), 2,000 of 1,590 12.9 vs 14.4, 20,000 of 1,020 52.9 vs 53.0; rows of
+// 32 nnz take 29 instructions in all (tiles 51).  FP64, beta = 0, us on the device
+// with 32 x 4 tiles and their fix-up and here: rows of lognormal length with
+// columns in runs, 4,284 of 2,640 nnz in the mean 33.0 and 27.9, 20,000 of 2,000 108
+// and 85; with random columns 5,000 x 2,000 nnz 48.5 and 44.0, 1,000 x 10,000 49.1
+// and 46.9, 20,000 x 1,100 102.7 and 89.2, one row of 10M 67.0 and 47.7, of 1M 10.6
+// and 10.9; lognormal with random columns, where L2's sectors bound both, 500 rows
+// of 3,000 12.7 and 11.0, 2,000 of 1,600 19.5 and 20.0, 4,284 of 2,640 55.1 and 58.4
+// (beta = 0.5: 59.7 and 58.5), 20,000 of 2,000 178 and 184 (187 and 184).  Rows of
 // 310 17.0 vs 14.8, and with FP32 storage no difference, so both keep the tiles.
+// Small matrices (a launch fewer): 60k power-law nnz 4.7 and 4.7 (beta = 0.5: 6.3
+// and 5.2), one row of 65,536 among 300 rows 6.6 and 5.6.
 // What bounds it: HBM on large matrices, the chain of column and x loads of a
-// piece on small ones.
+// piece on small ones.  The count is one atomic with release and acquire: with
+// fences around it 60k nnz took 5.0.
 #include <stdint.h>
 
 #include <algorithm>
@@ -30,20 +40,41 @@ namespace sbb {
 
 namespace {
 
-constexpr int NT = 256;  // threads per CTA
+constexpr int NT = 64;  // threads per CTA
 // Steps whose loads are in flight together, and the CTAs per SM that the launch
-// bounds aim at (40 registers).  12M nnz in 4,284 rows, us: 4 steps at 4, 5, 6 and
-// 7 CTAs 33.7, 33.8, 28.4, 37.3; 3 at 7 31.0; 6 at 5 32.3; 8 at 3 29.9.
+// bounds aim at (48 warps, 40 registers).  12M nnz in 4,284 rows, us, CTAs of 8
+// warps: 4 steps at 32, 40, 48 and 56 warps 33.7, 33.8, 28.4, 37.3; 3 at 56 31.0; 6
+// at 40 32.3; 8 at 24 29.9.  CTAs of 2 warps free their place sooner than of 8 and
+// spread evenly over the SMs: 5,000 x 2,000 nnz 44.4 and 50.2, 2,000 rows of 1,600
+// in pieces of 512 21.9 and 24.8.
 constexpr int kPieceSteps = 4;
-constexpr int kMinCtas = 6;
-// Piece sizes (multiples of 32): 1,024 nnz where that makes a piece for every
-// resident warp, smaller ones for smaller matrices (12M nnz, pieces of 512, 768,
-// 1,024, 2,048: 31.1, 30.8, 28.4, 36.8 us; 0.7M nnz, 512 and 1,024: 7.9, 10.8).
-// Pieces of groups of 8 lanes: 64 nnz.
-int piece_size(int nnz, int width)
+constexpr int kMinCtas = 24;
+constexpr int kSumSteps = 8;  // partial sums of a row that a lane loads together
+
+// Piece sizes, multiples of 32.  Of 32 lanes (`warps`: resident on the device): one
+// piece a row when the rows are short enough and fill the device; else, when
+// pieces of at most about 2,048 do, as many as fill 0.7 of it (3.3M nnz in 2,000
+// rows, pieces of 256, 512, 768, 1,024: 21.9, 21.9, 20.5, 21.5 us; 1.6M in 500,
+// 256, 384, 512, 1,024: 11.7, 11.5, 11.7, 13.3; 10M in 1,000, 768, 1,024, 2,048:
+// 51.8, 52.0, 47.5); else 1,024 (11M nnz in 4,284 rows, 512, 768, 1,024, 1,536,
+// 2,048: 29.7, 29.5, 27.9, 31.7, 31.8).  A row has at most kRowPieces8 or
+// kRowPieces32 pieces, whose sums one warp adds (a row of 65,536 nnz, 256, 512 and
+// 1,024 pieces of 8 lanes: 7.5, 6.1, 5.5 us).
+constexpr int kRowPieces8 = 1024, kRowPieces32 = 2048;
+int piece_size(int m, int nnz, int max_row, int width, long long warps)
 {
-    if (width == 8) return 64;
-    return nnz >= 1024 * 148 * 48 ? 1024 : (nnz >= 512 * 148 * 16 ? 512 : 256);
+    const int most = width == 8 ? kRowPieces8 : kRowPieces32;
+    long long size = 64;
+    if (width == 32) {
+        const double room = 0.7 * warps - 0.5 * m;
+        size = 1024;
+        if (max_row <= 2048 - 31 && m >= 0.7 * warps)
+            size = max_row + 31LL;
+        else if (room > 0 && nnz <= 2304.0 * room)
+            size = std::min(2048LL, std::max(256LL, (long long)(nnz / room)));
+    }
+    size = std::max(size, ((long long)max_row + most - 1) / most);
+    return (int)((size + 31) / 32 * 32);
 }
 
 struct PiecesPlan {
@@ -58,6 +89,18 @@ __device__ __forceinline__ int pieces_of(int lo, int hi, int size, int width)
 {
     const long long n = ((long long)hi - (lo & -width) + size - 1) / size;
     return n > 1 ? (int)n : 1;  // an empty row has one too: it writes beta*y
+}
+
+// One more piece of a row done: the count before it, which wraps to 0 after
+// `last`.  Release for this thread's partial sum, acquire for those counted.
+__device__ __forceinline__ unsigned ticket_take(unsigned *t, unsigned last)
+{
+    unsigned old;
+    asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "l"(t), "r"(last)
+                 : "memory");
+    return old;
 }
 
 // W lanes a piece; the 32 / W pieces of a warp run in step.
@@ -81,6 +124,13 @@ pieces_spmv_kernel(int n, int pieces, const int4 *__restrict__ piece,
     unsigned k = (first & -(unsigned)W) + sub, bad = 0;
     unsigned steps = (end - (first & -(unsigned)W) + W - 1) / W;
     if (W < 32) steps = __reduce_max_sync(0xffffffffu, steps);
+    // Of a row of several pieces: its ends, for the number of its pieces, on their
+    // way while the piece is read.
+    int row_lo = 0, row_hi = 0;
+    if (pc.w >= 0) {
+        row_lo = __ldg(rowptr + pc.x);
+        row_hi = __ldg(rowptr + pc.x + 1);
+    }
     ACC acc;
     acc.zero();
     int c[U];
@@ -118,28 +168,35 @@ pieces_spmv_kernel(int n, int pieces, const int4 *__restrict__ piece,
     double sum = acc.get();
 #pragma unroll
     for (int o = W / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, W);
-    if (pc.w < 0) {
-        if (sub == 0 && pc.x >= 0) write_y(y + pc.x, alpha, sum, beta, stream);
-        return;
-    }
-    // the lanes of a piece stay together from here
-    const unsigned mine = W == 32 ? 0xffffffffu : ((1u << (W & 31)) - 1u) << ((threadIdx.x & 31) / W * W);
-    const int np = pieces_of(__ldg(rowptr + pc.x), __ldg(rowptr + pc.x + 1), size, W);
-    unsigned done = 0;
-    if (sub == 0) {
+    if (sub == 0 && pc.w < 0 && pc.x >= 0) write_y(y + pc.x, alpha, sum, beta, stream);
+    if (!__any_sync(0xffffffffu, pc.w >= 0)) return;
+    const int np = pc.w >= 0 ? pieces_of(row_lo, row_hi, size, W) : 0;
+    bool last = false;
+    if (sub == 0 && pc.w >= 0) {
         __stcg(carry + i, sum);
-        __threadfence();
-        done = atomicInc(ticket + pc.w, (unsigned)np - 1u);
+        last = ticket_take(ticket + pc.w, (unsigned)np - 1u) == (unsigned)np - 1u;
     }
-    done = __shfl_sync(mine, done, 0, W);
-    if (done != (unsigned)np - 1u) return;
-    __threadfence();
-    sum = 0.0;
-#pragma unroll 4
-    for (int j = sub; j < np; j += W) sum += __ldcg(carry + pc.w + j);
+    // The sums of rows that are complete now; what the ticket ordered for the lane
+    // that took it holds for the whole warp.
+    unsigned rows = __ballot_sync(0xffffffffu, last);
+    while (rows) {
+        const int src = __ffs(rows) - 1;
+        rows &= rows - 1;
+        const int first_slot = __shfl_sync(0xffffffffu, pc.w, src);
+        const int count = __shfl_sync(0xffffffffu, np, src);
+        double total = 0.0;
+#pragma unroll 1
+        for (int j = threadIdx.x & 31; j < count; j += 32 * kSumSteps) {
+            double t[kSumSteps];
 #pragma unroll
-    for (int o = W / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(mine, sum, o, W);
-    if (sub == 0) write_y(y + pc.x, alpha, sum, beta, stream);
+            for (int u = 0; u < kSumSteps; ++u)
+                t[u] = j + 32 * u < count ? __ldcg(carry + first_slot + j + 32 * u) : 0.0;
+#pragma unroll
+            for (int u = 0; u < kSumSteps; ++u) total += t[u];
+        }
+        total = warp_sum(total);
+        if (sub == 0 && (threadIdx.x & 31) == src) write_y(y + pc.x, alpha, total, beta, stream);
+    }
 }
 
 // Numbers the pieces of every row, those of 32 consecutive rows in order, by a
@@ -176,6 +233,15 @@ pieces_list_kernel(const int *__restrict__ rowptr, int m, int size, int width,
     }
 }
 
+// Warps of the 32-lane form that the device holds at a time.
+long long resident_warps(bool f32)
+{
+    const LaunchShape ls =
+        f32 ? cached_launch_shape<pieces_spmv_kernel<ProdF32, AccF32, 32>>(NT, 0)
+            : cached_launch_shape<pieces_spmv_kernel<ProdF64, AccF64, 32>>(NT, 0);
+    return (long long)ls.sms * ls.occ * (NT / 32);
+}
+
 template <typename PT, typename ACC>
 void launch_pieces_t(const PiecesPlan &S, const Plan *p, double alpha, const void *x, double beta,
                      double *y, cudaStream_t s)
@@ -199,7 +265,7 @@ int pieces_build(Plan *p, cudaStream_t s)
     auto *S = new PiecesPlan();
     p->pieces = S;
     S->width = p->vector_width;
-    S->size = piece_size(p->nnz, S->width);
+    S->size = piece_size(p->m, p->nnz, p->max_row, S->width, resident_warps(p->f32));
     const long long cap = (long long)p->nnz / S->size + 2LL * p->m;
     if (cap > 0x7fffffffLL / 32) {
         set_error("row-piece plan: too many rows");
