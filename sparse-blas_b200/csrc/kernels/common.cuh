@@ -189,6 +189,20 @@ __device__ __forceinline__ void prefetch_l2(const void *a, size_t bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"(n) : "memory");
 }
 
+// Copies 4 bytes to shared memory without a register; copy_async_wait() waits
+// for all that the calling thread has started.
+__device__ __forceinline__ void copy_async(int *s, const int *g)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(s)),
+                 "l"(g)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // Programmatic dependent launch (sm_90+): a kernel launched with the
 // programmatic-serialization attribute may start before the kernel ahead of
 // it in the stream has finished; grid_dependency_wait() blocks until that

@@ -11,9 +11,10 @@
 //
 // Per warp segment (rows r0..r1-1 complete, row r1 open, nnz k0..k1-1):
 //   1. the products val*x of the segment's nnz go to the warp's shared memory
-//      and the row ends to its lanes: coalesced streaming loads of col/val, every
-//      load of the lane issued before any is used, x gathered through the
-//      read-only path with an L2 evict-last hint;
+//      and the row ends to its lanes, the 33rd and later ones to the shared memory
+//      behind the products: coalesced streaming loads of col/val, every load of
+//      the lane issued before any is used, x gathered through the read-only path
+//      with an L2 evict-last hint;
 //   2. each lane sums one row at a time straight from shared memory
 //      (consecutive lanes own consecutive rows, so the y writes coalesce);
 //      rows with more than kLongRow nnz in the segment are summed by the
@@ -27,7 +28,10 @@
 // matrices HBM's latency came first.  Predicated loads without branches, row ends
 // in registers and, on large matrices, several segments a warp with their nnz
 // brought into L2 together: 60M nnz 385 -> 282 us, 7.6M nnz 47.5 -> 43.1 (FP32
-// storage 44.2 -> 38.5), 1.1M nnz 12.3 -> 11.5.
+// storage 44.2 -> 38.5), 1.1M nnz 12.3 -> 11.5.  All row ends on their way at the
+// start, for segments of more than 32 rows: 1M rows of 0 to 4 nnz 26.2 -> 23.5 us
+// (24.6 with all ends in shared memory), 2M rows, half of them empty, 38.9 -> 32.8
+// (35.0), 7.6M nnz of a circuit 44.4 -> 40.3.
 #include <climits>
 
 #include "../sbb_internal.h"

@@ -239,6 +239,10 @@ __device__ __forceinline__ void merge_segments(
         }
         int end = k0;  // end of row r0 + b + lane, for the 32 rows from b
         if (lane < nrows) end = __ldg(rowptr + r0 + 1 + lane);
+        // the ends of further rows go behind the products, where there is room for
+        // one of each of the segment's items
+        int *s_end = reinterpret_cast<int *>(s_p + nz);
+        for (int i = 32 + lane; i < nrows; i += 32) copy_async(s_end + i, rowptr + r0 + 1 + i);
         double yv = 0.0;
         if (beta != 0.0 && lane < nrows) yv = ld_y(y + r0 + lane, streaming);
         V xv[IPT];
@@ -251,6 +255,7 @@ __device__ __forceinline__ void merge_segments(
 #pragma unroll
         for (int j = 0; j < IPT; ++j)
             if (lane + 32 * j < nz) s_p[lane + 32 * j] = PT::make(v[j], xv[j]);
+        if (nrows > 32) copy_async_wait();
         __syncwarp();
 
         // 2. complete rows r0 .. r1-1: lane per row, long rows by the warp
@@ -258,7 +263,7 @@ __device__ __forceinline__ void merge_segments(
         for (int b = 0; b < nrows; b += 32) {
             const int i = b + lane;
             if (b > 0) {
-                if (i < nrows) end = __ldg(rowptr + r0 + 1 + i);
+                if (i < nrows) end = s_end[i];
                 if (beta != 0.0 && i < nrows) yv = ld_y(y + r0 + i, streaming);
             }
             // a valid row pointer keeps 0 <= lo <= hi <= nz; clamping makes a
