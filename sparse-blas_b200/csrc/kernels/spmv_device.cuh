@@ -57,7 +57,7 @@ template <int V, int U> __device__ __forceinline__ double group_row_sums(double 
 // power-law rows of 30 with 16, 32 lanes 64, 44 (81, 54).  Without the bound on
 // the L2 prefetch rows of 100 took 42, without the loads ahead in a row 38.
 constexpr unsigned kVectorPrefetch = 256;
-template <typename PT, typename ACC, int V>
+template <typename PT, typename ACC, int V, bool AHEAD = true>
 __device__ __forceinline__ void vector_rows(int r0, int count, int n,
                                             const int *__restrict__ rowptr,
                                             const int *__restrict__ col,
@@ -79,6 +79,7 @@ __device__ __forceinline__ void vector_rows(int r0, int count, int n,
         }
     };
     auto prefetch = [&](int a, int b) {
+        if (!AHEAD) return;
         const unsigned first = (unsigned)__shfl_sync(0xffffffffu, a, 0);
         const unsigned end = __reduce_max_sync(0xffffffffu, (unsigned)b);
         if (lane == 0 && end - first - 1u < kVectorPrefetch) {
