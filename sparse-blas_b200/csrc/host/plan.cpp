@@ -354,6 +354,8 @@ static int plan_build_impl(Plan *p, const sbb_config *cfg, cudaStream_t s, bool 
         SBB_CUDA(cudaGetLastError());
         return SBB_OK;
     }
+    if (k == SBB_KERNEL_SLICED || k == SBB_KERNEL_PIECES)  // other kernels' shapes
+        p->ipt = p->persistent = p->tile_sigma = 0;
     if (k == SBB_KERNEL_SLICED) {
         const int w = c.vector_width;
         if (!validate || p->m > kTiledMaxRows || (w & (w - 1)) || w < 0 || w > 16) {
