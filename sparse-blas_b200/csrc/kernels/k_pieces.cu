@@ -14,7 +14,7 @@
 //
 // Why: on long rows the tiles' instructions (217 a 128-nnz tile) and L1 traffic
 // (76 % of its data pipe) come before HBM, and every tile carries its row on; here
-// 32 nnz take 29 instructions in all (tiles 51).  FP64, beta = 0, us on the device
+// 32 nnz take 32 instructions in all (tiles 51).  FP64, beta = 0, us on the device
 // with 32 x 4 tiles and their fix-up and here: rows of lognormal length with
 // columns in runs, 4,284 of 2,640 nnz in the mean 33.0 and 27.9, 20,000 of 2,000 108
 // and 85; with random columns 5,000 x 2,000 nnz 48.5 and 44.0, 1,000 x 10,000 49.1
@@ -82,6 +82,7 @@ struct PiecesPlan {
     int4 *piece = nullptr;       // row, first nnz, end, first slot of a row of several or -1
     double *carry = nullptr;     // partial sum of each piece of a row of several
     unsigned *ticket = nullptr;  // per row of several pieces (at its first slot): pieces done
+    int *count = nullptr;        // counters of the build
 };
 
 // Pieces of row [lo, hi), cut on multiples of `width` nnz.
@@ -176,9 +177,10 @@ pieces_spmv_kernel(int n, int pieces, const int4 *__restrict__ piece,
         __stcg(carry + i, sum);
         last = ticket_take(ticket + pc.w, (unsigned)np - 1u) == (unsigned)np - 1u;
     }
-    // The sums of rows that are complete now; what the ticket ordered for the lane
-    // that took it holds for the whole warp.
+    // The sums of rows that are complete now; with __syncwarp() what the ticket
+    // ordered for the lane that took it holds for the whole warp.
     unsigned rows = __ballot_sync(0xffffffffu, last);
+    __syncwarp();
     while (rows) {
         const int src = __ffs(rows) - 1;
         rows &= rows - 1;
@@ -271,30 +273,30 @@ int pieces_build(Plan *p, cudaStream_t s)
         set_error("row-piece plan: too many rows");
         return SBB_ERR_ARG;
     }
-    int *count = nullptr;
     auto al = [&](void **ptr, size_t bytes) {
         bytes = bytes ? bytes : 16;
         p->scratch_bytes += bytes;
         return dev_malloc_async(ptr, bytes, s) == cudaSuccess;
     };
-    if (!al((void **)&count, 4 * sizeof(int)) || !al((void **)&S->piece, sizeof(int4) * cap) ||
+    if (!al((void **)&S->count, 4 * sizeof(int)) || !al((void **)&S->piece, sizeof(int4) * cap) ||
         !al((void **)&S->carry, sizeof(double) * cap) ||
         !al((void **)&S->ticket, sizeof(unsigned) * cap)) {
         set_error("row-piece plan: device allocation failed");
         return SBB_ERR_NOMEM;
     }
-    SBB_CUDA(cudaMemsetAsync(count, 0, 4 * sizeof(int), s));
+    SBB_CUDA(cudaMemsetAsync(S->count, 0, 4 * sizeof(int), s));
     SBB_CUDA(cudaMemsetAsync(S->ticket, 0, sizeof(unsigned) * cap, s));
     if (p->m > 0) {
         const int grid = (int)std::min<long long>(((long long)p->m + 255) / 256, 148 * 16);
         pieces_list_kernel<<<grid, 256, 0, s>>>(p->rowptr, p->m, S->size, S->width, S->piece,
-                                            (int)cap, count);
-        launch_csr_check(p->rowptr, p->m, p->nnz, p->col, p->n, p->status, count + 2, s);
+                                            (int)cap, S->count);
+        launch_csr_check(p->rowptr, p->m, p->nnz, p->col, p->n, p->status, S->count + 2, s);
     }
-    SBB_CUDA(cudaMemcpyAsync(&S->pieces, count, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SBB_CUDA(cudaMemcpyAsync(&S->pieces, S->count, sizeof(int), cudaMemcpyDeviceToHost, s));
     SBB_CUDA(cudaStreamSynchronize(s));
     p->tiles = S->pieces;
-    SBB_CUDA(cudaFreeAsync(count, s));
+    SBB_CUDA(cudaFreeAsync(S->count, s));
+    S->count = nullptr;
     SBB_CUDA(cudaGetLastError());
     return SBB_OK;
 }
@@ -318,7 +320,7 @@ void pieces_free(Plan *p, cudaStream_t s)
 {
     auto *S = static_cast<PiecesPlan *>(p->pieces);
     if (!S) return;
-    for (void *q : {(void *)S->piece, (void *)S->carry, (void *)S->ticket})
+    for (void *q : {(void *)S->piece, (void *)S->carry, (void *)S->ticket, (void *)S->count})
         if (q) cudaFreeAsync(q, s);
     delete S;
     p->pieces = nullptr;
