@@ -345,8 +345,9 @@ int sbb_batch_create(sbb_batch_t *out, const sbb_batch_item *items, int count, v
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     for (int f = 0; f < kBatchFamilies; f++) {
         b->grid[f] = sms * std::max(batch_max_ctas_per_sm(f), 1);
-        // The grid's warps claim at least eight times each in the mean, so the
-        // last claims are a small part of the whole.  With 16 units of 1,024
+        // The grid's warps claim at least eight times each in the mean when there
+        // are that many units, so the last claims are a small part of the whole; with
+        // fewer a claim is one unit.  With 16 units of 1,024
         // nnz in every claim most warps had none or one: 30 matrices of up to
         // 8,000 rows took 875 us, 64 of up to 200,000 930 us; now 38 and 362.
         const long long warps = (long long)b->grid[f] * 8;

@@ -180,8 +180,10 @@ __device__ __forceinline__ void write_y(double *yp, double alpha, double sum, do
     st_y(yp, y_update(alpha, sum, beta, beta == 0.0 ? 0.0 : ld_y(yp, pol)), pol);
 }
 
-// Starts bringing [a, a + bytes) into L2 (whole 16-byte pieces around it: the
-// array must be 16-byte aligned and its allocation end on such a boundary).
+// Starts bringing [a, a + bytes) into L2, in whole 16-byte pieces: up to 15 bytes
+// before and behind it come along.  Nothing is read into the kernel, and a piece
+// that holds a byte of the array lies in a page of the array, so it is mapped
+// wherever the array starts and ends.
 __device__ __forceinline__ void prefetch_l2(const void *a, size_t bytes)
 {
     const uint64_t lo = reinterpret_cast<uint64_t>(a) & ~15ull;

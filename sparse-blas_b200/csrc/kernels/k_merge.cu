@@ -24,7 +24,7 @@
 // The reduction order depends only on the matrix and IPT, never on timing.
 //
 // What bounds it: the L1 data pipe (gathers, products and row sums through
-// shared memory) and issue, 440 instructions a 192-item segment (483 before); on large
+// shared memory) and issue, 449 instructions a 192-item segment (483 before); on large
 // matrices HBM's latency came first.  Predicated loads without branches, row ends
 // in registers and, on large matrices, several segments a warp with their nnz
 // brought into L2 together: 60M nnz 385 -> 282 us, 7.6M nnz 47.5 -> 43.1 (FP32

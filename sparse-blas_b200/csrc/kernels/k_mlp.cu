@@ -256,7 +256,7 @@ mlp_forward_kernel(const float *__restrict__ P, const float *__restrict__ X, int
 // 125 blocks hold 32 samples each, every stage is a register-tiled product
 // over shared memory, and the sums over blocks are left to
 // mlp_update_kernel: two launches and 17 us a step (12 us for 500 samples), bound by the latency of
-// its seven dependent stages (6.3 MFLOP a block).
+// its seven dependent stages (1.0 MFLOP a block).
 constexpr int kPartRow = (kParams + 1 + 31) / 32 * 32;
 __global__ void __launch_bounds__(MT)
 mlp_step_kernel(const float *__restrict__ P, const float *__restrict__ X, int N,

@@ -11,7 +11,7 @@
 // caller's row pointer; the copy is all that the plan adds.
 //
 // Why: the vector kernel reads the caller's arrays with V lanes a row, and on
-// short rows its issue slots (61 % used; 128 warp instructions per 24-nnz row,
+// short rows its issue slots (61 % used; 96 warp instructions per 24-nnz row,
 // most of them in the butterflies and the ragged ends of each row) and
 // latency come before HBM (24 %).  Here 32 nnz take 40 instructions in
 // all, 128 there.  Measured against it (FP64, beta = 0.5; us): 200k rows of 24

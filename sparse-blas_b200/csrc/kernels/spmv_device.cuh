@@ -55,7 +55,9 @@ template <int V, int U> __device__ __forceinline__ double group_row_sums(double 
 // a band with 8, 16, 32 lanes 18.6, 18.8, 25.5 (21.2, 21.4, 26.9 before); 100k
 // rows of 100 in blocks with 16, 32 lanes 30.9, 30.9 (36.1, 31.4); 100k
 // power-law rows of 30 with 16, 32 lanes 64, 44 (81, 54).  Without the bound on
-// the L2 prefetch rows of 100 took 42, without the loads ahead in a row 38.
+// the L2 prefetch rows of 100 took 42, without the loads ahead in a row 38.  Rows
+// of 150 with 32 lanes are no faster: 43.0 (42.5), FP32 storage 36.8 (35.9).
+// AHEAD: with the prefetches.
 constexpr unsigned kVectorPrefetch = 256;
 template <typename PT, typename ACC, int V, bool AHEAD = true>
 __device__ __forceinline__ void vector_rows(int r0, int count, int n,
