@@ -72,7 +72,8 @@ int get_row_from_index(int n, long long *a, long long idx);
 /* Replaces get_time (SparseBLAS/src/spmv_helper.cu:41-48): wall clock, s. */
 double get_time(void);
 /* Replaces get_gpu_availble_mem (SparseBLAS/src/spmv_helper.cu:51-76):
- * free memory in GB, minimum over the first ngpu devices that exist. */
+ * free memory in GB, minimum over the first ngpu devices that exist.  Memory
+ * that the library keeps between calls counts as free and is given back. */
 double get_gpu_availble_mem(int ngpu);
 
 /* ========================= Part 2: device API ============================ */
@@ -100,7 +101,8 @@ enum {
                               for short, even rows (vector_width: W = 1, 2, 4,
                               8 or 16, 0 = from mean row length).  No
                               counterpart in the reference. */
-    SBB_KERNEL_PIECES = 7, /* K6: rows in pieces of at most 64 to 1,024 nnz,
+    SBB_KERNEL_PIECES = 7, /* K6: rows in pieces of at most 64 to 2,048 nnz (more
+                              in rows of millions),
                               vector_width (8 or 32, 0 = 32) lanes each, from
                               the caller's arrays (no copy); for long rows and
                               small matrices.  No counterpart in the
