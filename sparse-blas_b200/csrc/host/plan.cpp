@@ -43,12 +43,12 @@ int plan_launches(const Plan *p)
 // Lanes per row of the row slices: enough that a row takes about 8 to 32 steps
 // (us for 1, 2, 4, 8 lanes: rows of 6 11.8, 12.4, 15.7, -; of 24 15.5, 14.4,
 // 15.8, 19.0; of 50 -, 15.4, 15.0, 16.3; of 100 -, 27.1, 26.4, 26.6), and more
-// while the slices are fewer than an SM's warps times the SMs (3,000 rows of 24:
-// 5.3, 3.6, 2.8, 2.4).
-static int slice_width(int m, double mean)
+// while the slices are fewer than the kernel's 48 warps an SM times the SMs (3,000
+// rows of 24: 5.3, 3.6, 2.8, 2.4).
+static int slice_width(int m, double mean, int sms)
 {
     int w = mean <= 8 ? 1 : (mean <= 32 ? 2 : (mean <= 128 ? 4 : 8));
-    while (w < 8 && w < mean && (long long)m * w / 32 < 148 * 48) w <<= 1;
+    while (w < 8 && w < mean && (long long)m * w / 32 < 48LL * sms) w <<= 1;
     return w;
 }
 
@@ -194,7 +194,8 @@ static int build_sliced(Plan *p, int width, bool fall_back, cudaStream_t s)
 {
     const int vw = p->vector_width;
     const size_t bytes = p->scratch_bytes;
-    p->vector_width = width ? width : slice_width(p->m, p->m > 0 ? (double)p->nnz / p->m : 0.0);
+    const double mean = p->m > 0 ? (double)p->nnz / p->m : 0.0;
+    p->vector_width = width ? width : slice_width(p->m, mean, sm_count(p->device));
     int rc = sliced_build(p, s);
     if (rc == SBB_OK) {
         unsigned st = 0;
