@@ -7,6 +7,7 @@
 
 using sbb::lane_reach;
 using sbb::lane_share;
+using sbb::lane_step;
 
 static int failures = 0;
 static void check(bool ok, const char *what, unsigned a, unsigned b)
@@ -31,6 +32,15 @@ int main()
                     check(most == len - li, "nnz of the long row", most, li);
                     unsigned long long off = (most - 1) / v * (unsigned long long)v;
                     check(off < most && off + v >= most, "last step", most, v);
+                    // the short row's own index, any number of steps on and one ahead
+                    unsigned k = last - own + li, taken = 0;
+                    for (int i = 0; i < 1000; i++) {
+                        taken += k < last;
+                        check(k + v > k, "index wraps", k, v);
+                        k = lane_step(k, last, v);
+                    }
+                    check(taken == (own && li == 0) && lane_step(k, last, v) == k,
+                          "short row by index", taken, li);
                     for (int i = 0; i < 3; i++, off += v)  // it, and two more loaded ahead
                         check(off <= 0xffffffffull && (unsigned)off >= reach, "walks again", li, v);
                 }
