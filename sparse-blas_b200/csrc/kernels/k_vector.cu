@@ -48,9 +48,10 @@ template <typename PT, typename ACC, int V>
 void launch_vector_v(const CsrView &A, double alpha, const typename PT::V *x, double beta,
                      double *y, unsigned *status, cudaStream_t s)
 {
-    // Without prefetches for FP32 storage when a warp has several chunks to run
-    // ahead with (1M rows of 38 122.9 us with them, 117.8 without; 30,000 of 60, a
-    // chunk a warp, 8.4 and 8.9).
+    // FP32 storage when a warp has several chunks: nothing runs ahead in a row or
+    // into L2 (us with both, with neither: 1M rows of 38 120.9 and 108.7, 1.3M of 2
+    // 19.1 and 18.4, 100,000 of 150 37.9 and 37.3; 30,000 of 60, a chunk a warp, 8.4
+    // and 8.9).
     constexpr bool kAhead = sizeof(typename PT::V) == 8;
     constexpr auto kern = vector_kernel<PT, ACC, V, true>;
     constexpr auto plain = vector_kernel<PT, ACC, V, kAhead>;

@@ -56,8 +56,8 @@ template <int V, int U> __device__ __forceinline__ double group_row_sums(double 
 // rows of 100 in blocks with 16, 32 lanes 30.9, 30.9 (36.1, 31.4); 100k
 // power-law rows of 30 with 16, 32 lanes 64, 44 (81, 54).  Without the bound on
 // the L2 prefetch rows of 100 took 42, without the loads ahead in a row 38.  Rows
-// of 150 with 32 lanes are no faster: 43.0 (42.5), FP32 storage 36.8 (35.9).
-// AHEAD: with the prefetches.
+// of 150 with 32 lanes are no faster: 43.0 (42.5), FP32 storage 37.3 (35.9).
+// AHEAD: with the prefetches and the loads ahead in a row.
 constexpr unsigned kVectorPrefetch = 256;
 template <typename PT, typename ACC, int V, bool AHEAD = true>
 __device__ __forceinline__ void vector_rows(int r0, int count, int n,
@@ -114,18 +114,35 @@ __device__ __forceinline__ void vector_rows(int r0, int count, int n,
         hi = nhi;
         if (at + 2 * CR < count) load_rows(at + 2 * CR, nlo, nhi);
         int c[U];
-        T v[U];
+        T v[U], xv[U];
+        auto load = [&](unsigned off) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            c[u] = ld_stream_if(col + k[u], 0u < reach[u]);
-            v[u] = ld_stream_if(val + k[u], 0u < reach[u]);
-        }
-        // FP64: an index per row; FP32 storage: one offset for all (the other way round,
-        // us: 9 small matrices as a batch 32.8 and 32.0, FP32 rows of 150 38.4 and 36.9)
-        if constexpr (sizeof(T) == 8) {
+            for (int u = 0; u < U; ++u) {
+                c[u] = ld_stream_if(col + (k[u] + off), off < reach[u]);
+                v[u] = ld_stream_if(val + (k[u] + off), off < reach[u]);
+            }
+        };
+        auto gather = [&](unsigned off) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) xv[u] = gather_x_if(x, c[u], n, off < reach[u], bad);
+        };
+        if constexpr (!AHEAD) {
+#pragma unroll 1
+            for (unsigned off = 0; off < most; off += V) {
+                load(off);
+                gather(off);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (off < reach[u]) acc[u].mac(v[u], xv[u]);
+            }
+        } else if constexpr (sizeof(T) == 8) {
+            // FP64: an index per row; FP32 storage: one offset for all (the other way
+            // round, us: 9 small matrices as a batch 32.8 and 32.0, FP32 rows of 150 38.4
+            // and 36.9)
+            load(0);
             bool any = most > 0;
             while (any) {
-                T xv[U], vn[U];
+                T vn[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) xv[u] = gather_x_if(x, c[u], n, k[u] < end[u], bad);
                 any = false;
@@ -146,11 +163,11 @@ __device__ __forceinline__ void vector_rows(int r0, int count, int n,
                 }
             }
         } else {
+            load(0);
 #pragma unroll 1
             for (unsigned off = 0; off < most; off += V) {
-                T xv[U], vn[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) xv[u] = gather_x_if(x, c[u], n, off < reach[u], bad);
+                T vn[U];
+                gather(off);
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const bool p = off + V < reach[u];
