@@ -39,7 +39,7 @@ cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
 // Memory that the pool holds and nothing uses.
 size_t pool_idle_bytes();
 // After the frees that end a plan or a call, enqueued on s: when the pool holds
-// more than its bound, waits for them, and the excess goes back to the device.
+// more than its bound unused, waits for them, and the excess goes back to the device.
 void pool_settle(cudaStream_t s);
 // Gives what the current device's pool holds unused back to the device; returns
 // the bytes of it whose frees have yet to be synchronised with.
